@@ -257,28 +257,16 @@ __device__ __forceinline__ void batch_problem(const BatchDev &b, BatchShared &sh
                     sv[v][2] = (T)src[i2];
                     sv[v][3] = (T)src[i3];
                 }
-                bool fallback = false;
-                T vm_rho = T(0), vp_rho = T(0);
-#pragma unroll
-                for (int v = 0; v < 7; ++v) {
-                    const T a0 = sv[v][0], a1 = sv[v][1], a2 = sv[v][2], a3 = sv[v][3], a4 = sv[v][4];
-                    T vm, vp;
-                    recon_cell<T, REC>(w, a0, a1, a2, a3, a4, vm, vp);
-                    if (v == 0) { vm_rho = vm; vp_rho = vp; }
-                    if (v == 4 && b.pos_fallback) {
-                        fallback = !(vm_rho > T(0) && vp_rho > T(0) && vm > T(0) && vp > T(0));
-                        if (fallback) {
-                            for (int u = 0; u < 4; ++u) {
-                                const T cv = sv[u][2];  // (T)P[u][i2]
-                                if (c0 <= n) QL[u][c] = cv;
-                                if (c0 >= 1) QR[u][c - 1] = cv;
-                            }
-                        }
-                    }
-                    if (fallback) vm = vp = a2;
+                auto at = [&](int v, int m) -> T { return sv[v][m + 2]; };
+                auto again = [&](int v, int m) -> T {
+                    const double *src = (v < 5) ? b.P[v] : b.BC[v == 5 ? 1 : 2];
+                    return (T)src[cl(c0 + m)];
+                };
+                auto put = [&](int v, T vm, T vp) {
                     if (c0 <= n) QL[v][c] = vp;
                     if (c0 >= 1) QR[v][c - 1] = vm;
-                }
+                };
+                recon_all<T, REC, 0>(w, false, b.pos_fallback, nullptr, at, again, put);
             }
             gsync(coop);
             // ---- B: Riemann solve on faces 0..n, then the edge EMFs there ----
@@ -293,10 +281,8 @@ __device__ __forceinline__ void batch_problem(const BatchDev &b, BatchShared &sh
                 pl[ibx] = bn;
                 pr[ibx] = bn;
                 const T g = (T)b.gamma;
-                const T epsL = eos_eps(pl[irho], pl[itau], g), epsR = eos_eps(pr[irho], pr[itau], g);
-                const T csL = eos_cs(pl[itau], pl[irho], epsL, g), csR = eos_cs(pr[itau], pr[irho], epsR, g);
                 T fo[9];
-                riemann_face<T, 0, RS>(pl, pr, epsL, epsR, csL, csR, fo);
+                face_flux<T, 0, RS>(pl, pr, g, fo);
 #pragma unroll
                 for (int v = 0; v < 5; ++v) b.F[v][c] = (double)fo[1 + v];
                 // edge EMFs (mhd_module.f90:310-432 in 1D): face EMFs from the

@@ -71,6 +71,12 @@ struct Dev {
     double *EX, *EY, *EZ;  // edge EMFs
     void *QL[7], *QR[7];   // face states of the split flux path (double or float)
 
+    // faces of the FP64 HLLD form left to k_faces_deferred: their two states
+    // (16 arrays of fix_cap), 3 * cell + direction, and how many
+    double *fix;
+    unsigned *fix_at, *fix_n;
+    unsigned fix_cap;
+
     // grid metrics (getgrid.f90), offsets: cells +2, faces +3
     const double *x, *dx, *xF, *xbar, *dx_cb;
     const double *y, *dy, *yF, *sine, *sinf, *dcose, *dsine;
@@ -119,6 +125,7 @@ __device__ __forceinline__ void unflat3(unsigned t, unsigned ex, unsigned ey, in
 
 // host-side launchers of the face-flux kernels (one per precision unit)
 void launch_flux_fp64(const Dev &d, int dir, int rec, int rs, dim3 grid, dim3 block, size_t smem, cudaStream_t s);
+void launch_faces_deferred(const Dev &d, cudaStream_t s);
 void launch_flux_fp32(const Dev &d, int dir, int rec, int rs, dim3 grid, dim3 block, size_t smem, cudaStream_t s);
 void launch_split_fp64(const Dev &d, int dir, int rec, int rs, cudaStream_t s, const TmaMaps *tma = nullptr);
 void launch_split_fp32(const Dev &d, int dir, int rec, int rs, cudaStream_t s);

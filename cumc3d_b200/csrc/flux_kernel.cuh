@@ -19,6 +19,7 @@
 // exactly one thread.
 #pragma once
 #include "engine.cuh"
+#include "fast64.cuh"
 #include "mhd_device.cuh"
 
 namespace cumc {
@@ -33,10 +34,154 @@ __device__ __forceinline__ T eos_cs(T p, T rho, T e, T g) {
     return dsqrt(dpdden + dpdint * p / (rho * rho));
 }
 
+// One face from its two primitive states: the face EOS, BUILDSTATES and the
+// solver, with the plain arithmetic.
+template <class T, int DIR, int RS>
+__device__ __forceinline__ void face_flux_plain(const T *pl, const T *pr, T g, T *fo) {
+    const T epsL = eos_eps(pl[irho], pl[itau], g);
+    const T epsR = eos_eps(pr[irho], pr[itau], g);
+    const T csL = eos_cs(pl[itau], pl[irho], epsL, g);
+    const T csR = eos_cs(pr[itau], pr[irho], epsR, g);
+    riemann_face<T, DIR, RS>(pl, pr, epsL, epsR, csL, csR, fo);
+}
+template <int DIR>
+__device__ __noinline__ void hlld_out_of_line(const double *q, double g, double *fo) {
+    double pl[9], pr[9];
+#pragma unroll
+    for (int i = 1; i <= 8; ++i) {
+        pl[i] = q[i];
+        pr[i] = q[8 + i];
+    }
+    face_flux_plain<double, DIR, RS_HLLD>(pl, pr, g, fo);
+}
+// The same, FP64 HLLD through hlld64 (fast64.cuh); a face it does not vouch for
+// is solved again with the plain form, out of line so that its registers and
+// its divisions' branches stay out of the common path.
+template <class T, int DIR, int RS>
+__device__ __forceinline__ void face_flux(const T *pl, const T *pr, T g, T *fo) {
+    if constexpr (sizeof(T) == sizeof(double) && RS == RS_HLLD) {
+        if (!hlld64<DIR>(pl, pr, g, fo)) {
+            double q[17], f[9];
+#pragma unroll
+            for (int i = 1; i <= 8; ++i) {
+                q[i] = pl[i];
+                q[8 + i] = pr[i];
+            }
+            hlld_out_of_line<DIR>(q, g, f);
+#pragma unroll
+            for (int i = 1; i <= 8; ++i) fo[i] = f[i];
+        }
+    } else {
+        face_flux_plain<T, DIR, RS>(pl, pr, g, fo);
+    }
+}
+
+template <class T> __device__ __forceinline__ void store_flux(double *a, int i, T v);
+
+// fluxes and MHD_FLUX (mhd_module.f90:229-270) of one face
+template <class T, int DIR>
+__device__ __forceinline__ void store_face(const Dev &d, int ci, const T *fo) {
+    double *const *FO = (DIR == 0) ? d.FX : (DIR == 1) ? d.FY : d.FZ;
+#pragma unroll
+    for (int v = 0; v < 5; ++v) store_flux<T>(FO[v], ci, fo[1 + v]);
+    if (DIR == 0) {
+        d.EF[e_yx][ci] = (double)fo[ibz];
+        d.EF[e_zx][ci] = -(double)fo[iby];
+    } else if (DIR == 1) {
+        d.EF[e_xy][ci] = -(double)fo[ibz];
+        d.EF[e_zy][ci] = (double)fo[ibx];
+    } else {
+        d.EF[e_xz][ci] = (double)fo[iby];
+        d.EF[e_yz][ci] = -(double)fo[ibx];
+    }
+}
+
+// Solve the face at ci and store it.  A face that hlld64 does not vouch for
+// goes on the stage's list, which k_faces_deferred works off after the sweeps:
+// about one face in a hundred where fields decay towards zero (products
+// between 1e-323 and 1e-271), but spread so that the plain form inside this
+// kernel ran in most warps (spherical torus 124 x 44 x 128, the three sweeps
+// of a step: 1.45 ms that way, 0.87 with the list).  A full list falls back to
+// the plain form here.
+template <class T, int DIR, int RS>
+__device__ __forceinline__ void solve_face(const Dev &d, int ci, const T *pl, const T *pr) {
+    T fo[9];
+    if constexpr (sizeof(T) == sizeof(double) && RS == RS_HLLD) {
+        if (!hlld64<DIR>(pl, pr, d.gamma, fo)) {
+            const unsigned slot = atomicAdd(d.fix_n, 1u);
+            double q[17];
+#pragma unroll
+            for (int i = 1; i <= 8; ++i) {
+                q[i] = pl[i];
+                q[8 + i] = pr[i];
+            }
+            if (slot < d.fix_cap) {
+#pragma unroll
+                for (int i = 1; i <= 16; ++i) d.fix[(size_t)(i - 1) * d.fix_cap + slot] = q[i];
+                d.fix_at[slot] = 3u * (unsigned)ci + DIR;
+                return;
+            }
+            double f[9];
+            hlld_out_of_line<DIR>(q, d.gamma, f);
+            store_face<double, DIR>(d, ci, f);
+            return;
+        }
+    } else {
+        face_flux_plain<T, DIR, RS>(pl, pr, (T)d.gamma, fo);
+    }
+    store_face<T, DIR>(d, ci, fo);
+}
+
+// The seven variables of one cell: at(v, m) is the value of variable v at
+// stencil position m = -2..2, put(v, vm, vp) takes its left and right edge.
+// A cell whose edge density or pressure is not positive falls back to first
+// order where the option asks for it (the reference has no such guard); count
+// is where such a cell is counted, if anywhere.  FAST: FP64 WENO-Z through
+// weno64; returns whether every variable stands.  Otherwise the plain forms.
+template <class T, int REC, int UNI, bool FAST, int UNROLL, class At, class Put>
+__device__ __forceinline__ bool recon_vars(const T *__restrict__ w, bool linear, int pos_fallback,
+                                           unsigned long long *count, At at, Put put) {
+    constexpr bool WIDE = REC == REC_PPM || REC == REC_WENO;
+    T vm_rho = T(0), vp_rho = T(0);
+    bool fallback = false, ok = true;
+#pragma unroll UNROLL
+    for (int v = 0; v < 7; ++v) {
+        T a0 = T(0), a4 = T(0);
+        if (WIDE) { a0 = at(v, -2); a4 = at(v, 2); }
+        const T a1 = at(v, -1), a2 = at(v, 0), a3 = at(v, 1);
+        T vm, vp;
+        if (REC == REC_WENO && linear) weno_linear<T>(w, a0, a1, a2, a3, a4, vm, vp);
+        else if constexpr (FAST) ok &= weno64<UNI != 0>(w, a0, a1, a2, a3, a4, vm, vp);
+        else recon_cell<T, REC>(w, a0, a1, a2, a3, a4, vm, vp);
+        if (v == 0) { vm_rho = vm; vp_rho = vp; }
+        if (v == 4 && pos_fallback) {
+            fallback = !(vm_rho > T(0) && vp_rho > T(0) && vm > T(0) && vp > T(0));
+            if (fallback) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) put(u, at(u, 0), at(u, 0));
+            }
+        }
+        if (fallback) vm = vp = a2;
+        put(v, vm, vp);
+    }
+    if (fallback && ok && count) atomicAdd(count, 1ull);
+    return ok;
+}
+// again: at() for a second pass of a cell, where it differs
+template <class T, int REC, int UNI, class At, class Again, class Put>
+__device__ __forceinline__ void recon_all(const T *__restrict__ w, bool linear, int pos_fallback,
+                                          unsigned long long *count, At at, Again again, Put put) {
+    if constexpr (sizeof(T) == sizeof(double) && REC == REC_WENO) {
+        if (!recon_vars<T, REC, UNI, true, 7>(w, linear, pos_fallback, count, at, put))
+            recon_vars<T, REC, UNI, false, 1>(w, linear, pos_fallback, count, again, put);
+    } else {
+        recon_vars<T, REC, UNI, false, 7>(w, linear, pos_fallback, count, at, put);
+    }
+}
+
 // hydro face fluxes are stored in the precision of the flux arithmetic: FP64
 // in the plain form, FP32 in the FP32 form (the RK accumulation that reads
 // them stays FP64); the arrays are FP64-sized either way
-template <class T> __device__ __forceinline__ void store_flux(double *a, int i, T v);
 template <> __device__ __forceinline__ void store_flux<double>(double *a, int i, double v) { a[i] = v; }
 template <> __device__ __forceinline__ void store_flux<float>(double *a, int i, float v) {
     reinterpret_cast<float *>(a)[i] = v;
@@ -124,39 +269,13 @@ __global__ void __launch_bounds__(256) k_flux(const Dev d) {
         constexpr int NW = (REC == REC_PPM) ? 14 : (REC == REC_WENO) ? 10 : 2;
 #pragma unroll
         for (int m = 0; m < NW; ++m) w[m] = wp[m];
-        bool fallback = false;
-#pragma unroll
-        for (int v = 0; v < 7; ++v) {
-            const T *sv = sS + v * SR * SX + sb;
-            T a0 = T(0), a4 = T(0);
-            if (REC == REC_PPM || REC == REC_WENO) {
-                a0 = sv[-2 * sm];
-                a4 = sv[2 * sm];
-            }
-            T a1 = sv[-sm];
-            T a2 = sv[0];
-            T a3 = sv[sm];
-            T vm, vp;
-            recon_cell<T, REC>(w, a0, a1, a2, a3, a4, vm, vp);
-            if (v == 4 && d.pos_fallback) {
-                // first-order fallback when an edge density or pressure is not
-                // positive (optional; the reference has no such guard)
-                fallback = !(sVM[0 * nthr + tid] > T(0) && sVP[0 * nthr + tid] > T(0) && vm > T(0) && vp > T(0));
-                // a cell shared by two tiles (ls = TS - 1 and 0 of the next) counts once
-                if (fallback && d.fb_count && (ls < TS - 1 || c == ns + 1)) atomicAdd(d.fb_count, 1ull);
-                if (fallback) {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const T cv = sS[u * SR * SX + sb];
-                        sVM[u * nthr + tid] = cv;
-                        sVP[u * nthr + tid] = cv;
-                    }
-                }
-            }
-            if (fallback) vm = vp = a2;
+        auto at = [&](int v, int m) -> T { return sS[v * SR * SX + sb + m * sm]; };
+        auto put = [&](int v, T vm, T vp) {
             sVM[v * nthr + tid] = vm;
             sVP[v * nthr + tid] = vp;
-        }
+        };
+        // a cell shared by two tiles (ls = TS - 1 and 0 of the next) counts once
+        recon_all<T, REC, 0>(w, false, d.pos_fallback, (ls < TS - 1 || c == ns + 1) ? d.fb_count : nullptr, at, at, put);
     }
     __syncthreads();
     if (!(rvalid && ls < TS - 1 && c <= ns)) return;
@@ -176,28 +295,7 @@ __global__ void __launch_bounds__(256) k_flux(const Dev d) {
     const T bn = (T)d.P[F::ibn - 1][ci];  // face field at face c (ppmc_module.f90:198-199)
     pl[F::ibn] = bn;
     pr[F::ibn] = bn;
-    const T g = (T)d.gamma;
-    const T epsL = eos_eps(pl[irho], pl[itau], g);
-    const T epsR = eos_eps(pr[irho], pr[itau], g);
-    const T csL = eos_cs(pl[itau], pl[irho], epsL, g);
-    const T csR = eos_cs(pr[itau], pr[irho], epsR, g);
-    T fo[9];
-    riemann_face<T, DIR, RS>(pl, pr, epsL, epsR, csL, csR, fo);
-
-    double *const *FO = (DIR == 0) ? d.FX : (DIR == 1) ? d.FY : d.FZ;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) store_flux<T>(FO[v], ci, fo[1 + v]);
-    // MHD_FLUX, solver/mhd/mhd_module.f90:229-270
-    if (DIR == 0) {
-        d.EF[e_yx][ci] = (double)fo[ibz];
-        d.EF[e_zx][ci] = -(double)fo[iby];
-    } else if (DIR == 1) {
-        d.EF[e_xy][ci] = -(double)fo[ibz];
-        d.EF[e_zy][ci] = (double)fo[ibx];
-    } else {
-        d.EF[e_xz][ci] = (double)fo[iby];
-        d.EF[e_yz][ci] = -(double)fo[ibx];
-    }
+    solve_face<T, DIR, RS>(d, ci, pl, pr);
 }
 
 // ---------------------------------------------------------------------------
@@ -215,7 +313,7 @@ template <> __device__ __forceinline__ float uni_w<float>(const Dev &d, int dir,
 // along this axis, checked bit for bit on the host); they then come from the
 // kernel parameters and live in uniform registers.
 template <class T, int DIR, int REC, int UNI>
-__global__ void __launch_bounds__(256) k_recon(const Dev d) {
+__global__ void __launch_bounds__(256, sizeof(T) == 8 && REC == REC_WENO ? 2 : 1) k_recon(const Dev d) {
     if (d.S->done) return;
     // one thread per reconstructed cell, enumerated x fastest with no tail
     // padding per row: x extent nx+2 (x sweep) or nx, then y, then z
@@ -248,38 +346,15 @@ __global__ void __launch_bounds__(256) k_recon(const Dev d) {
     }
     T *const *QL = reinterpret_cast<T *const *>(d.QL);
     T *const *QR = reinterpret_cast<T *const *>(d.QR);
-    T vm_rho = T(0), vp_rho = T(0);
-    bool fallback = false;
-#pragma unroll
-    for (int v = 0; v < 7; ++v) {
+    auto at = [&](int v, int m) -> T {
         const double *src = (v < 5) ? d.P[v] : d.BC[v == 5 ? tb1 : tb2];
-        T a0 = T(0), a4 = T(0);
-        if (REC == REC_PPM || REC == REC_WENO) {
-            a0 = (T)__ldg(src + ci - 2 * st);
-            a4 = (T)__ldg(src + ci + 2 * st);
-        }
-        T a1 = (T)__ldg(src + ci - st);
-        T a2 = (T)__ldg(src + ci);
-        T a3 = (T)__ldg(src + ci + st);
-        T vm, vp;
-        recon_cell<T, REC>(w, a0, a1, a2, a3, a4, vm, vp);
-        if (v == 0) { vm_rho = vm; vp_rho = vp; }
-        if (v == 4 && d.pos_fallback) {
-            fallback = !(vm_rho > T(0) && vp_rho > T(0) && vm > T(0) && vp > T(0));
-            if (fallback && d.fb_count) atomicAdd(d.fb_count, 1ull);
-            if (fallback) {
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const T cv = (T)__ldg(d.P[u] + ci);
-                    if (c <= ns) QL[u][ci] = cv;
-                    if (c >= 1) QR[u][ci - st] = cv;
-                }
-            }
-        }
-        if (fallback) vm = vp = a2;
+        return (T)__ldg(src + ci + m * st);
+    };
+    auto put = [&](int v, T vm, T vp) {
         if (c <= ns) QL[v][ci] = vp;       // left state of face c
         if (c >= 1) QR[v][ci - st] = vm;   // right state of face c-1
-    }
+    };
+    recon_all<T, REC, UNI>(w, false, d.pos_fallback, d.fb_count, at, at, put);
 }
 
 template <class T, int DIR, int RS, int MINB>
@@ -318,26 +393,7 @@ __global__ void __launch_bounds__(128, MINB) k_riemann(const Dev d) {
     const T bn = (T)d.P[F::ibn - 1][ci];
     pl[F::ibn] = bn;
     pr[F::ibn] = bn;
-    const T g = (T)d.gamma;
-    const T epsL = eos_eps(pl[irho], pl[itau], g);
-    const T epsR = eos_eps(pr[irho], pr[itau], g);
-    const T csL = eos_cs(pl[itau], pl[irho], epsL, g);
-    const T csR = eos_cs(pr[itau], pr[irho], epsR, g);
-    T fo[9];
-    riemann_face<T, DIR, RS>(pl, pr, epsL, epsR, csL, csR, fo);
-    double *const *FO = (DIR == 0) ? d.FX : (DIR == 1) ? d.FY : d.FZ;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) store_flux<T>(FO[v], ci, fo[1 + v]);
-    if (DIR == 0) {
-        d.EF[e_yx][ci] = (double)fo[ibz];
-        d.EF[e_zx][ci] = -(double)fo[iby];
-    } else if (DIR == 1) {
-        d.EF[e_xy][ci] = -(double)fo[ibz];
-        d.EF[e_zy][ci] = (double)fo[ibx];
-    } else {
-        d.EF[e_xz][ci] = (double)fo[iby];
-        d.EF[e_yz][ci] = -(double)fo[ibx];
-    }
+    solve_face<T, DIR, RS>(d, ci, pl, pr);
 }
 
 // The Riemann kernel with its loads taken off the critical path: CTAs of 128
@@ -407,26 +463,7 @@ __global__ void __launch_bounds__(128, MINB) k_riemann_pf(const Dev d) {
         const T bn = (T)bb[b][tid];
         pl[F::ibn] = bn;
         pr[F::ibn] = bn;
-        const T g = (T)d.gamma;
-        const T epsL = eos_eps(pl[irho], pl[itau], g);
-        const T epsR = eos_eps(pr[irho], pr[itau], g);
-        const T csL = eos_cs(pl[itau], pl[irho], epsL, g);
-        const T csR = eos_cs(pr[itau], pr[irho], epsR, g);
-        T fo[9];
-        riemann_face<T, DIR, RS>(pl, pr, epsL, epsR, csL, csR, fo);
-        double *const *FO = (DIR == 0) ? d.FX : (DIR == 1) ? d.FY : d.FZ;
-#pragma unroll
-        for (int v = 0; v < 5; ++v) store_flux<T>(FO[v], ci, fo[1 + v]);
-        if (DIR == 0) {
-            d.EF[e_yx][ci] = (double)fo[ibz];
-            d.EF[e_zx][ci] = -(double)fo[iby];
-        } else if (DIR == 1) {
-            d.EF[e_xy][ci] = -(double)fo[ibz];
-            d.EF[e_zy][ci] = (double)fo[ibx];
-        } else {
-            d.EF[e_xz][ci] = (double)fo[iby];
-            d.EF[e_yz][ci] = -(double)fo[ibx];
-        }
+        solve_face<T, DIR, RS>(d, ci, pl, pr);
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
@@ -449,15 +486,20 @@ static inline void split_dims(const Dev &d, int dir, bool recon, dim3 &g, dim3 &
 #include "recon_tile.cuh"
 namespace cumc {
 
-template <class T, int DIR, int UNI, int CPT, int MINB = 1>
+// KIND: the recon_tile choice (1, 2, 4)
+template <class T, int DIR, int UNI, int CPT, int KIND>
 static void launch_recon_tile_c(const Dev &d, int rec, cudaStream_t s) {
     const dim3 g = recon_tile_grid(d, DIR, CPT), b(32, 8, 1);
+    // blocks per SM: FP64 WENO-Z unrolls to 250 registers where nothing bounds
+    // it; 2 blocks (126 registers) and, as kind 4, 3 blocks (80, 152 B spilled)
+    constexpr bool W = sizeof(T) == sizeof(double);
+    constexpr int M = KIND == 4 ? 4 : 1, MW = !W ? M : KIND == 4 ? 3 : 2;
     switch (rec) {
-        case REC_TVD_MM: k_recon_tile<T, DIR, REC_TVD_MM, UNI, CPT, 0, MINB><<<g, b, 0, s>>>(d); break;
-        case REC_TVD_VL: k_recon_tile<T, DIR, REC_TVD_VL, UNI, CPT, 0, MINB><<<g, b, 0, s>>>(d); break;
-        case REC_TVD_MC: k_recon_tile<T, DIR, REC_TVD_MC, UNI, CPT, 0, MINB><<<g, b, 0, s>>>(d); break;
-        case REC_PPM: k_recon_tile<T, DIR, REC_PPM, UNI, CPT, 0, MINB><<<g, b, 0, s>>>(d); break;
-        default: k_recon_tile<T, DIR, REC_WENO, UNI, CPT, 0, MINB><<<g, b, 0, s>>>(d); break;
+        case REC_TVD_MM: k_recon_tile<T, DIR, REC_TVD_MM, UNI, CPT, 0, M><<<g, b, 0, s>>>(d); break;
+        case REC_TVD_VL: k_recon_tile<T, DIR, REC_TVD_VL, UNI, CPT, 0, M><<<g, b, 0, s>>>(d); break;
+        case REC_TVD_MC: k_recon_tile<T, DIR, REC_TVD_MC, UNI, CPT, 0, M><<<g, b, 0, s>>>(d); break;
+        case REC_PPM: k_recon_tile<T, DIR, REC_PPM, UNI, CPT, 0, M><<<g, b, 0, s>>>(d); break;
+        default: k_recon_tile<T, DIR, REC_WENO, UNI, CPT, 0, MW><<<g, b, 0, s>>>(d); break;
     }
 }
 // recon_tile: 1, 2 staged tiles with 1 or 2 cells per thread; 4 one cell per
@@ -465,9 +507,9 @@ static void launch_recon_tile_c(const Dev &d, int rec, cudaStream_t s) {
 // where no tensor maps are given
 template <class T, int DIR, int UNI>
 static void launch_recon_tile(const Dev &d, int rec, cudaStream_t s) {
-    if (d.recon_tile == 2) launch_recon_tile_c<T, DIR, UNI, 2>(d, rec, s);
+    if (d.recon_tile == 2) launch_recon_tile_c<T, DIR, UNI, 2, 2>(d, rec, s);
     else if (d.recon_tile == 4) launch_recon_tile_c<T, DIR, UNI, 1, 4>(d, rec, s);
-    else launch_recon_tile_c<T, DIR, UNI, 1>(d, rec, s);
+    else launch_recon_tile_c<T, DIR, UNI, 1, 1>(d, rec, s);
 }
 
 template <class T, int DIR, int UNI>

@@ -145,37 +145,15 @@ __device__ __forceinline__ void recon_tile_cells(const Dev &d, const T *__restri
 #pragma unroll
             for (int m = 0; m < NW; ++m) w[m] = wp[m];
         }
-        T vm_rho = T(0), vp_rho = T(0);
-        bool fallback = false;
-#pragma unroll
-        for (int v = 0; v < 7; ++v) {
-            // the stencil c-H .. c+H of variable v
-            auto at = [&](int m) -> T {
-                return (DIR == 0) ? s[v * SLOT + r * SX + tx + HO + m] : s[v * SLOT + (r + HO + m) * SX + tx + XO];
-            };
-            T a0 = T(0), a4 = T(0);
-            if (H == 2) { a0 = at(-2); a4 = at(2); }
-            const T a1 = at(-1), a2 = at(0), a3 = at(1);
-            T vm, vp;
-            if (LRN && linear) weno_linear<T>(w, a0, a1, a2, a3, a4, vm, vp);
-            else recon_cell<T, REC>(w, a0, a1, a2, a3, a4, vm, vp);
-            if (v == 0) { vm_rho = vm; vp_rho = vp; }
-            if (v == 4 && d.pos_fallback) {
-                fallback = !(vm_rho > T(0) && vp_rho > T(0) && vm > T(0) && vp > T(0));
-                if (fallback && d.fb_count) atomicAdd(d.fb_count, 1ull);
-                if (fallback) {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const T cv = (DIR == 0) ? s[u * SLOT + r * SX + tx + HO] : s[u * SLOT + (r + HO) * SX + tx + XO];
-                        if (c <= ns) QL[u][ci] = cv;
-                        if (c >= 1) QR[u][ci - st] = cv;
-                    }
-                }
-            }
-            if (fallback) vm = vp = a2;
+        // the stencil c-H .. c+H of variable v
+        auto at = [&](int v, int m) -> T {
+            return (DIR == 0) ? s[v * SLOT + r * SX + tx + HO + m] : s[v * SLOT + (r + HO + m) * SX + tx + XO];
+        };
+        auto put = [&](int v, T vm, T vp) {
             if (c <= ns) QL[v][ci] = vp;      // left state of face c
             if (c >= 1) QR[v][ci - st] = vm;  // right state of face c-1
-        }
+        };
+        recon_all<T, REC, UNI>(w, LRN && linear, d.pos_fallback, d.fb_count, at, at, put);
     }
 }
 
