@@ -32,6 +32,7 @@
 
 #include "../../include/cumc3d_gpu.h"
 #include "engine.cuh"
+#include "fast64.cuh"
 #include "learned.cuh"
 #include "mhd_device.cuh"
 #include "poisson.cuh"
@@ -314,25 +315,66 @@ __global__ void k_snapshot_pack(const Dev d, double *__restrict__ out) {
 // ---------------------------------------------------------------------------
 // du/dt and the Shu-Osher combination over j,k,l = 0..n
 // ---------------------------------------------------------------------------
-// l_operator face-B induction of one face component, spatial.f90:639-702
-// (x: from the z edges at k, k-1 and the y edges at l, l-1; y and z alike)
-__device__ __forceinline__ double lr_face_x(const Dev &d, int j, int k, int l, double ez0, double ezy, double ey0,
-                                           double eyz) {
-    if (d.coord == 0) return -(dv(ez0 - ezy, DY(k)) - dv(ey0 - eyz, DZ(l)));
-    if (d.coord == 1) return dv(-(ez0 - ezy), XF(j) * DY(k)) + dv(ey0 - eyz, DZ(l));
-    return (-(SINF(k) * ez0 - SINF(k - 1) * ezy) + (ey0 - eyz) * (DY(k) / DZ(l))) / (XF(j) * DCOSE(k) + small_num);
+// The divisors of one cell's update: FLUX_DIFF's three (h) and the induction's
+// (fa, fb per face component), each reciprocal formed once for the 15 + 6
+// quotients (on Cartesian axes the same three serve all).  With a division
+// apiece the arithmetic of this memory-bound kernel took longer than its loads
+// (256^3, FP64: 4.08 ms a step; 3.05 with shared reciprocals and 3 blocks per
+// SM: 168 registers, no spills -- 4, 5 and 6 blocks took 3.81, 4.07, 4.52).
+struct CellDens {
+    Den64 h[3], fa[3], fb[3];
+};
+template <int COORD>
+__device__ __forceinline__ CellDens cell_dens(const Dev &d, int j, int k, int l) {
+    CellDens q;
+    if (COORD == 0) {
+        const Den64 x = den64(DX(j)), y = den64(DY(k)), z = den64(DZ(l));
+        q = {{x, y, z}, {y, z, x}, {z, x, y}};
+    } else if (COORD == 1) {
+        const Den64 x = den64(XC(j) * DX(j)), y = den64(XC(j) * DY(k)), z = den64(DZ(l));
+        q = {{x, y, z}, {den64(XF(j) * DY(k)), z, x}, {z, den64(DX(j)), y}};
+    } else {
+        const Den64 x = den64(XC(j) * DX(j));
+        q = {{den64(DXCB(j) / 3.0), den64(XBAR(j) * DCOSE(k)), den64(XBAR(j) * DZ(l) * DCOSE(k))},
+             {den64(XF(j) * DCOSE(k) + small_num), den64(XBAR(j) * SINF(k) * DZ(l) + small_num), x},
+             {x, x, den64(XBAR(j) * DY(k))}};
+    }
+    return q;
 }
-__device__ __forceinline__ double lr_face_y(const Dev &d, int j, int k, int l, double ex0, double exz, double ez0,
-                                           double ezx) {
-    if (d.coord == 0) return -(dv(ex0 - exz, DZ(l)) - dv(ez0 - ezx, DX(j)));
-    if (d.coord == 1) return dv(-(ex0 - exz), DZ(l)) + dv(ez0 - ezx, DX(j));
-    return (-(ex0 - exz) / (XBAR(j) * SINF(k) * DZ(l) + small_num) + (XF(j) * ez0 - XF(j - 1) * ezx) / (XC(j) * DX(j)));
-}
-__device__ __forceinline__ double lr_face_z(const Dev &d, int j, int k, int l, double ey0, double eyx, double ex0,
-                                           double exy) {
-    if (d.coord == 0) return -(dv(ey0 - eyx, DX(j)) - dv(ex0 - exy, DY(k)));
-    if (d.coord == 1) return dv(-(XF(j) * ey0 - XF(j - 1) * eyx), XC(j) * DX(j)) + dv(ex0 - exy, XC(j) * DY(k));
-    return (-(XF(j) * ey0 - XF(j - 1) * eyx) / (XC(j) * DX(j)) + (ex0 - exy) / (XBAR(j) * DY(k)));
+
+// l_operator face-B induction of face component a, spatial.f90:639-702 (x: from
+// the z edges at k, k-1 and the y edges at l, l-1; y and z alike): e0 - e0m and
+// e1 - e1m the differences of the two edge EMFs, in that order
+template <int COORD>
+__device__ __forceinline__ double lr_face(const Dev &d, const CellDens &q, int a, int j, int k, int l, double e0,
+                                          double e0m, double e1, double e1m) {
+    double n0, n1;
+    if (COORD == 0) {
+        n0 = e0 - e0m;
+        n1 = e1 - e1m;
+    } else if (COORD == 1) {
+        n0 = a == 2 ? -(XF(j) * e0 - XF(j - 1) * e0m) : -(e0 - e0m);
+        n1 = e1 - e1m;
+    } else if (a == 0) {
+        n0 = -(SINF(k) * e0 - SINF(k - 1) * e0m) + (e1 - e1m) * (DY(k) / DZ(l));
+        n1 = 0.0;
+    } else if (a == 1) {
+        n0 = -(e0 - e0m);
+        n1 = XF(j) * e1 - XF(j - 1) * e1m;
+    } else {
+        n0 = -(XF(j) * e0 - XF(j - 1) * e0m);
+        n1 = e1 - e1m;
+    }
+    bool ok = true;
+    double r0 = over(n0, q.fa[a], ok), r1 = 0.0;
+    const bool two = !(COORD == 2 && a == 0);
+    if (two) r1 = over(n1, q.fb[a], ok);
+    if (!ok) {
+        r0 = n0 / q.fa[a].b;
+        if (two) r1 = n1 / q.fb[a].b;
+    }
+    if (!two) return r0;
+    return COORD == 0 ? -(r0 - r1) : r0 + r1;
 }
 
 // the Shu-Osher combination of one variable, rungekutta.f90:61-167
@@ -342,12 +384,26 @@ __device__ __forceinline__ double rk_combine(int stage, double u, double u0, dou
     return rk30 * u0 + rk31 * u + rk32 * dt * lr;
 }
 
+// -n0/h0 - n1/h1 - n2/h2 over the grid's dimensions
+__device__ __forceinline__ double flux_diff(int n_dim, const double *n, const Den64 *h) {
+    bool ok = true;
+    double L = -over(n[0], h[0], ok);
+    if (n_dim > 1) L = L - over(n[1], h[1], ok);
+    if (n_dim > 2) L = L - over(n[2], h[2], ok);
+    if (!ok) {
+        L = -(n[0] / h[0].b);
+        if (n_dim > 1) L = L - n[1] / h[1].b;
+        if (n_dim > 2) L = L - n[2] / h[2].b;
+    }
+    return L;
+}
+
 // FLUX_DIFF + sources + the face-B induction + the Shu-Osher combination of
 // one cell (j,k,l in 0..n): un = the cell's new conserved state; in stage 1
 // the old state is saved to u_old.  (Hydro components of the index-0 layers
 // are combined with a zero operator, as the reference leaves them undefined
 // and never reads them back.)
-template <class FT>
+template <class FT, int COORD>
 __device__ __forceinline__ void rk_cell(const Dev &d, int stage, int j, int k, int l, int c, double *un) {
     const int sy = d.NX, sz = d.NX * d.NY;
     const bool interior = (j >= 1 && k >= 1 && l >= 1);
@@ -379,37 +435,29 @@ __device__ __forceinline__ void rk_cell(const Dev &d, int stage, int j, int k, i
     }
     const double dt = d.S->dt;
     double lr[8];
+    const CellDens q = cell_dens<COORD>(d, j, k, l);
     if (interior) {
         // FLUX_DIFF, spatial.f90:436-583
 #pragma unroll
         for (int i = 0; i < 5; ++i) {
-            double dflux, L;
-            if (d.coord == 0) dflux = dv(fx0[i] - fx1[i], DX(j));
-            else if (d.coord == 1) dflux = dv(XF(j) * fx0[i] - XF(j - 1) * fx1[i], XC(j) * DX(j));
-            else dflux = dv(XF(j) * XF(j) * fx0[i] - XF(j - 1) * XF(j - 1) * fx1[i], DXCB(j) / 3.0);
-            L = -dflux;
-            if (d.n_dim > 1) {
-                if (d.coord == 0) dflux = dv(fy0[i] - fy1[i], DY(k));
-                else if (d.coord == 1) dflux = dv(fy0[i] - fy1[i], XC(j) * DY(k));
-                else dflux = dv(SINF(k) * fy0[i] - SINF(k - 1) * fy1[i], XBAR(j) * DCOSE(k));
-                L = L - dflux;
-            }
-            if (d.n_dim > 2) {
-                if (d.coord != 2) dflux = dv(fz0[i] - fz1[i], DZ(l));
-                else dflux = dv((fz0[i] - fz1[i]) * DY(k), XBAR(j) * DZ(l) * DCOSE(k));
-                L = L - dflux;
-            }
+            double n[3];
+            n[0] = COORD == 0 ? fx0[i] - fx1[i]
+                   : COORD == 1 ? XF(j) * fx0[i] - XF(j - 1) * fx1[i]
+                                  : XF(j) * XF(j) * fx0[i] - XF(j - 1) * XF(j - 1) * fx1[i];
+            n[1] = COORD != 2 ? fy0[i] - fy1[i] : SINF(k) * fy0[i] - SINF(k - 1) * fy1[i];
+            n[2] = COORD != 2 ? fz0[i] - fz1[i] : (fz0[i] - fz1[i]) * DY(k);
+            const double L = flux_diff(d.n_dim, n, q.h);
             lr[i] = L;
         }
         // GET_SOURCE (spatial.f90:191-256) + CUSTOM_SOURCE
         double sc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-        const bool need_prim = d.coord != 0 || d.source_kind != 0;
+        const bool need_prim = COORD != 0 || d.source_kind != 0;
         if (need_prim) {
             const double rho = d.P[0][c], vx = d.P[1][c], vy = d.P[2][c], vz = d.P[3][c], p = d.P[4][c];
-            if (d.coord != 0) {
+            if (COORD != 0) {
                 const double bx = d.BC[0][c], by = d.BC[1][c], bz = d.BC[2][c];
                 const double bsquare = bx * bx + by * by + bz * bz;
-                if (d.coord == 1) {
+                if (COORD == 1) {
                     sc[1] = sc[1] + dv(p + rho * vy * vy + 0.5 * bsquare - by * by, XC(j));
                     sc[2] = sc[2] - dv(rho * vx * vy - bx * by, XC(j));
                 } else {
@@ -468,9 +516,9 @@ __device__ __forceinline__ void rk_cell(const Dev &d, int stage, int j, int k, i
         for (int i = 0; i < 5; ++i) lr[i] = 0.0;  // undefined in the reference, never read back
     }
     // l_operator face-B induction, spatial.f90:639-702
-    lr[5] = lr_face_x(d, j, k, l, ez0, ezy, ey0, eyz);
-    lr[6] = lr_face_y(d, j, k, l, ex0, exz, ez0, ezx);
-    lr[7] = lr_face_z(d, j, k, l, ey0, eyx, ex0, exy);
+    lr[5] = lr_face<COORD>(d, q, 0, j, k, l, ez0, ezy, ey0, eyz);
+    lr[6] = lr_face<COORD>(d, q, 1, j, k, l, ex0, exz, ez0, ezx);
+    lr[7] = lr_face<COORD>(d, q, 2, j, k, l, ey0, eyx, ex0, exy);
     // rungekutta.f90:61-167
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -479,8 +527,8 @@ __device__ __forceinline__ void rk_cell(const Dev &d, int stage, int j, int k, i
     }
 }
 
-template <class FT>  // storage type of the hydro face fluxes (double, or float in the FP32 form)
-__global__ void __launch_bounds__(128, 4) k_rk(const Dev d, int stage) {
+template <class FT, int COORD>  // storage type of the hydro face fluxes (double, or float in the FP32 form)
+__global__ void __launch_bounds__(128, 3) k_rk(const Dev d, int stage) {
     if (d.S->done) return;
     // flat index over j,k,l = 0..n (x fastest)
     // (64-bit index arithmetic: the 32-bit form, cheaper in instructions,
@@ -494,7 +542,7 @@ __global__ void __launch_bounds__(128, 4) k_rk(const Dev d, int stage) {
     const int l = (int)(r / ey);
     const int c = cidx(d, j, k, l);
     double un[8];
-    rk_cell<FT>(d, stage, j, k, l, c, un);
+    rk_cell<FT, COORD>(d, stage, j, k, l, c, un);
 #pragma unroll
     for (int i = 0; i < 8; ++i) d.U[i][c] = un[i];
 }
@@ -547,19 +595,19 @@ __global__ void __launch_bounds__(256, 2) k_rk_cart(const Dev d, int stage) {
     }
     const double dt = d.S->dt;
     double lr[8];
+    const CellDens q = cell_dens<0>(d, j, k, l);  // Cartesian here: three reciprocals
 #pragma unroll
     for (int i = 0; i < 5; ++i) {
         lr[i] = 0.0;
         if (interior) {
-            double L = -dv((double)f[i][0] - (double)f[i][1], DX(j));
-            if (d.n_dim > 1) L = L - dv((double)f[i][2] - (double)f[i][3], DY(k));
-            if (d.n_dim > 2) L = L - dv((double)f[i][4] - (double)f[i][5], DZ(l));
-            lr[i] = L + 0.0;
+            const double n[3] = {(double)f[i][0] - (double)f[i][1], (double)f[i][2] - (double)f[i][3],
+                                 (double)f[i][4] - (double)f[i][5]};
+            lr[i] = flux_diff(d.n_dim, n, q.h) + 0.0;
         }
     }
-    lr[5] = -(dv(ez0 - ezy, DY(k)) - dv(ey0 - eyz, DZ(l)));
-    lr[6] = -(dv(ex0 - exz, DZ(l)) - dv(ez0 - ezx, DX(j)));
-    lr[7] = -(dv(ey0 - eyx, DX(j)) - dv(ex0 - exy, DY(k)));
+    lr[5] = lr_face<0>(d, q, 0, j, k, l, ez0, ezy, ey0, eyz);
+    lr[6] = lr_face<0>(d, q, 1, j, k, l, ex0, exz, ez0, ezx);
+    lr[7] = lr_face<0>(d, q, 2, j, k, l, ey0, eyx, ex0, exy);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         double un;
@@ -635,12 +683,23 @@ __device__ __forceinline__ void recover_cell(const Dev &d, int stage, int j, int
         cell_b(d, j, k, l, bfx, ux_m, bfy, uy_m, bfz, uz_m, bc);
         const double u0 = u_c[0];
         rho = u0;
-        vx = dv(u_c[1], u0);
-        vy = dv(u_c[2], u0);
-        vz = dv(u_c[3], u0);
         const double bsquare = bc[0] * bc[0] + bc[1] * bc[1] + bc[2] * bc[2];
+        const double ne = u_c[4] - 0.5 * bsquare;
+        // one reciprocal for the four quotients
+        const Den64 r = den64(u0);
+        bool ok = true;
+        vx = over(u_c[1], r, ok);
+        vy = over(u_c[2], r, ok);
+        vz = over(u_c[3], r, ok);
+        e = over(ne, r, ok);
+        if (!ok) {
+            vx = u_c[1] / u0;
+            vy = u_c[2] / u0;
+            vz = u_c[3] / u0;
+            e = ne / u0;
+        }
         const double vsquare = vx * vx + vy * vy + vz * vz;
-        e = (u_c[4] - 0.5 * bsquare) / u0 - 0.5 * vsquare;
+        e = e - 0.5 * vsquare;
     } else {
         rho = d.P[0][c]; vx = d.P[1][c]; vy = d.P[2][c]; vz = d.P[3][c];
         e = d.EPS[c];
@@ -688,7 +747,15 @@ __device__ __forceinline__ void recover_cell(const Dev &d, int stage, int j, int
         dpdrho = d.eps_floor * g1;
         dpdeps = d.rho_floor * g1;
     }
-    const double cs = sqrt(dpdrho + dpdeps * p / (rho * rho));
+    const double r2 = rho * rho, np = dpdeps * p;
+    const Den64 dr2 = den64(r2);
+    bool ok = true;
+    double a2 = dpdrho + over(np, dr2, ok);
+    double cs = sqrt64(a2);
+    if (!(ok & in_pos(a2, -200, 200))) {
+        a2 = dpdrho + np / r2;
+        cs = sqrt(a2);
+    }
     d.P[0][c] = rho;
     d.P[1][c] = vx;
     d.P[2][c] = vy;
@@ -1384,6 +1451,13 @@ static void enqueue_stage_a(cumc_handle *h, int stage) {
     launch_fills(h, true);
     prof_end(h, PC_EMF);
 }
+template <class FT>
+static void launch_rk(const Dev &d, int stage, long long cells, cudaStream_t s) {
+    const unsigned g = (unsigned)((cells + 127) / 128);
+    if (d.coord == 0) k_rk<FT, 0><<<g, 128, 0, s>>>(d, stage);
+    else if (d.coord == 1) k_rk<FT, 1><<<g, 128, 0, s>>>(d, stage);
+    else k_rk<FT, 2><<<g, 128, 0, s>>>(d, stage);
+}
 static void enqueue_stage_b(cumc_handle *h, int stage) {
     Range r("cumc stage: edge EMFs + update + recovery + ghosts");
     const Dev &d = h->d;
@@ -1404,9 +1478,9 @@ static void enqueue_stage_b(cumc_handle *h, int stage) {
         if (fp32 && d.coord == 0 && d.source_kind == 0 && cells < (1LL << 31)) {
             k_rk_cart<float><<<(unsigned)((cells + 255) / 256), 256, 0, h->stream>>>(d, stage);
         } else if (fp32) {
-            k_rk<float><<<(unsigned)((cells + 127) / 128), 128, 0, h->stream>>>(d, stage);
+            launch_rk<float>(d, stage, cells, h->stream);
         } else {
-            k_rk<double><<<(unsigned)((cells + 127) / 128), 128, 0, h->stream>>>(d, stage);
+            launch_rk<double>(d, stage, cells, h->stream);
         }
     }
     h->launches++;

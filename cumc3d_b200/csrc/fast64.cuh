@@ -101,6 +101,21 @@ __device__ __forceinline__ bool sum_ok(double s, double n1, double n2) {
 // the low word of an all-ones mantissa
 __device__ __forceinline__ bool not_ones(double b) { return lo64(b) != 0xFFFFFFFFu; }
 
+// A positive divisor shared by several quotients.  over() is x / b where its
+// test holds; ok collects the tests, and where one fails the caller divides
+// again with the plain form.
+struct Den64 {
+    double b, y;
+    bool ok;
+};
+__device__ __forceinline__ Den64 den64(double b) {
+    return {b, inv64(b), in_pos(b, -60, 60) & not_ones(b)};
+}
+__device__ __forceinline__ double over(double x, const Den64 &d, bool &ok) {
+    ok &= d.ok & num_ok(x);
+    return quo(x, d.b, d.y);
+}
+
 // ---------------------------------------------------------------------------
 // WENO-Z (weno of mhd_device.cuh, the same roundings).  Products by powers of
 // two are exact, so they are folded into fused multiply-adds: with
