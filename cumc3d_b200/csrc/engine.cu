@@ -5,22 +5,23 @@
 // as the kernel sequence
 //
 //   k_flux x/y/z        recon + EOS + BUILDSTATES + Riemann + MHD_FLUX      (flux_kernel.cuh)
-//   k_ecell             cell EMF + the 1D/2D face-EMF fill                  (mhd_module.f90:310-356)
-//   k_ebnd x/y/z        BOUNDARY_EFIELD                                     (mhd_module.f90:478-840)
-//   k_edge              edge EMFs (GS05 arithmetic average)                 (mhd_module.f90:364-432)
+//   k_edge              the 1D/2D face-EMF fill, BOUNDARY_EFIELD and the
+//                       edge EMFs (GS05 arithmetic average)                 (mhd_module.f90:314-432,
+//                                                                            478-840)
 //   k_fixpole           FIXPOLE axis average (spherical only)               (mhd_module.f90:437-461)
 //   k_rk                FLUX_DIFF + GET_SOURCE + CUSTOM_SOURCE + l_operator
 //                       + the Shu-Osher stage combination                   (spatial.f90:167-713,
 //                                                                            rungekutta.f90:61-167)
 //   k_rk_cart           the same for the FP32 form on Cartesian grids without sources
 //   k_recover           FROMUTORVE + CUSTOM_CHECKRHO + FROMRVETOU
-//                       + FINDPRESSURE on the interior                       (fromrvetou.f90, update.f90)
-//   k_cons0             FROMRVETOU on the index-0 ghost layer (face fields)
-//   k_bnd x/y/z         BOUNDARY (prim, bcell, epsilon, p, c_s)              (boundary.f90:5-770)
-//   k_custom_bc         CUSTOM_BOUNDARY_X/Z of the torus models
+//                       + FINDPRESSURE on the interior, the next stage's
+//                       cell EMFs                                            (fromrvetou.f90, update.f90,
+//                                                                            mhd_module.f90:310-312)
+//   k_ghosts            BOUNDARY (prim, bcell, epsilon, p, c_s) and the
+//                       torus models' CUSTOM_BOUNDARY_X/Z                    (boundary.f90:5-770)
 //
-// FINDDT is a deterministic min-reduction (exact, order independent) whose
-// result stays on the device; a whole step is captured once as a CUDA graph
+// FINDDT is a deterministic min-reduction (exact, order independent; inside
+// cumc_evolve by the last stage's k_recover) whose result stays on the device; a whole step is captured once as a CUDA graph
 // and replayed by cumc_evolve.
 #include <cmath>
 #include <cstdio>
@@ -66,45 +67,7 @@ __device__ __forceinline__ void set_error(const Dev &d, int code, int cell, int 
 }
 
 // ---------------------------------------------------------------------------
-// cell EMFs + the 1D/2D face-EMF assignment, mhd_module.f90:310-356
-// ---------------------------------------------------------------------------
-__global__ void k_ecell(const Dev d) {
-    if (d.S->done) return;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int k = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    const int l = blockIdx.z + 1;
-    if (j > d.nx || k > d.ny || l > d.nz) return;
-    const int c = cidx(d, j, k, l);
-    const double vx = d.P[1][c], vy = d.P[2][c], vz = d.P[3][c];
-    const double bx = d.BC[0][c], by = d.BC[1][c], bz = d.BC[2][c];
-    const double ex = vz * by - vy * bz;
-    const double ey = vx * bz - vz * bx;
-    const double ez = vy * bx - vx * by;
-    d.EC[0][c] = ex;
-    d.EC[1][c] = ey;
-    d.EC[2][c] = ez;
-    if (d.n_dim == 1) {
-        const int c0y = cidx(d, j, 0, 1), c0z = cidx(d, j, 1, 0);
-        d.EF[e_xy][c] = ex;
-        d.EF[e_zy][c] = ez;
-        d.EF[e_xy][c0y] = ex;
-        d.EF[e_zy][c0y] = ez;
-        d.EF[e_xz][c] = ex;
-        d.EF[e_yz][c] = ey;
-        d.EF[e_xz][c0z] = ex;
-        d.EF[e_yz][c0z] = ey;
-    } else if (d.n_dim == 2) {
-        const int c0z = cidx(d, j, k, 0);
-        d.EF[e_xz][c] = ex;
-        d.EF[e_yz][c] = ey;
-        d.EF[e_xz][c0z] = ex;
-        d.EF[e_yz][c0z] = ey;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// ghost fills.  Each pass covers one axis for every cell of the other two
-// padded axes, exactly like the reference's sequential x -> y -> z loops.
+// ghost fills
 // ---------------------------------------------------------------------------
 // source index of ghost layer g (1..3) on one side of an axis with n cells
 __device__ __forceinline__ int ghost_src(int flag, bool inner, int g, int n) {
@@ -116,125 +79,210 @@ __device__ __forceinline__ int ghost_src(int flag, bool inner, int g, int n) {
     return inner ? g : n + 1 - g;         // reflect/axis/equator (parity applied by caller)
 }
 
-struct FillList {
-    double *a[16];
-    signed char par[16];  // parity factor, 0 = plain copy
-    int n;
+// the thirteen arrays of BOUNDARY: P 0..4, cell B, P 5..7, c_s, epsilon
+struct GhostList {
+    double *a[13];
+    unsigned char axes[13];  // bit x: the fill of axis x covers the array
+    unsigned char var[13];   // parity index
 };
+constexpr int GHOST_GROUPS = 4;  // blockIdx.y: arrays 0-3, 4-7, 8-10, 11-12
 
-__device__ __forceinline__ void fill_one(const FillList &fl, int dst, int src, bool parity) {
-#pragma unroll 4
-    for (int m = 0; m < fl.n; ++m) {
-        double v = fl.a[m][src];
-        if (parity) v = (double)fl.par[m] * v;
-        fl.a[m][dst] = v;
-    }
-}
-
-// AXIS: 0 x, 1 y, 2 z.  Thread grid: (other0 padded) x (other1 padded) x 3 layers.
-template <int AXIS>
-__global__ void k_fill(const Dev d, const FillList in_list, const FillList out_list, int eps_out_mode) {
+// BOUNDARY (boundary.f90:5-770) and CUSTOM_BOUNDARY_X/Z (torus velocity clamps,
+// model/torus-cyn/src/custom.f90:146-208) in one pass over the ghost cells.  The
+// reference fills x, then y, then z; every fill is a copy times a parity, so a
+// ghost cell's value is that of the cell its indices map to axis by axis, and
+// an array a fill leaves out (the normal face field) keeps its index there.
+// No source is itself written: on every axis that moves it is an interior index.
+// Three dependent passes and the clamps took four launches a stage.
+__global__ void __launch_bounds__(256) k_ghosts(const Dev d, const GhostList gl) {
     if (d.S->done) return;
-    int o0 = blockIdx.x * blockDim.x + threadIdx.x;  // fastest remaining axis, padded index
-    int o1 = blockIdx.y;
-    int g = blockIdx.z + 1;
-    int n, flag_in, flag_out, dstride;
+    unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    // cells with a ghost index in x, then in y, then in z only
+    const unsigned n0 = 6u * d.NY * d.NZ, n1 = 6u * d.nx * d.NZ, n2 = 6u * d.nx * d.ny;
+    auto layer = [](unsigned g, int n) { return g < 3 ? (int)g - 2 : n + (int)g - 2; };
     int j, k, l;
-    if (AXIS == 0) {
-        if (o0 >= d.NY) return;
-        k = o0 - 2; l = o1 - 2; j = 0;
-        n = d.nx; flag_in = d.bf[0]; flag_out = d.bf[1]; dstride = 1;
-    } else if (AXIS == 1) {
-        if (o0 >= d.NX) return;
-        j = o0 - 2; l = o1 - 2; k = 0;
-        n = d.ny; flag_in = d.bf[2]; flag_out = d.bf[3]; dstride = d.NX;
+    if (t < n0) {
+        int g;
+        unflat3(t, 6u, (unsigned)d.NY, g, k, l);
+        j = layer(g, d.nx);
+        k -= 2;
+        l -= 2;
+    } else if ((t -= n0) < n1) {
+        int g;
+        unflat3(t, (unsigned)d.nx, 6u, j, g, l);
+        ++j;
+        k = layer(g, d.ny);
+        l -= 2;
+    } else if ((t -= n1) < n2) {
+        int g;
+        unflat3(t, (unsigned)d.nx, (unsigned)d.ny, j, k, g);
+        ++j;
+        ++k;
+        l = layer(g, d.nz);
     } else {
-        if (o0 >= d.NX) return;
-        j = o0 - 2; k = o1 - 2; l = 0;
-        n = d.nz; flag_in = d.bf[4]; flag_out = d.bf[5]; dstride = d.NX * d.NY;
+        return;
     }
-    const int base = cidx(d, j, k, l);  // index of position 0 along AXIS
-    // inner side
-    {
-        int s = ghost_src(flag_in, true, g, n);
-        fill_one(in_list, base + (1 - g) * dstride, base + s * dstride, flag_in >= 2);
-    }
-    // outer side
-    {
-        int s = ghost_src(flag_out, false, g, n);
-        fill_one(out_list, base + (n + g) * dstride, base + s * dstride, flag_out >= 2);
-    }
-    // epsilon with the BOUNDARY1D_NM y-outer rule (boundary.f90:243-282)
-    if (AXIS == 1 && eps_out_mode >= 0) {
-        int s = ghost_src(eps_out_mode, false, g, n);
-        double v = d.EPS[base + s * dstride];
-        d.EPS[base + (n + g) * dstride] = v;  // epsilon is even on every side
-    }
-}
-
-// CUSTOM_BOUNDARY_X/Z: torus velocity clamps (model/torus-cyn/src/custom.f90:146-208)
-__global__ void k_custom_bc(const Dev d) {
-    if (d.S->done) return;
-    const int o0 = blockIdx.x * blockDim.x + threadIdx.x;
-    const int o1 = blockIdx.y;
-    const int g = blockIdx.z + 1;
-    if (o0 < d.NY && o1 < d.NZ) {  // x ghosts: (k = o0-2, l = o1-2)
-        const int k = o0 - 2, l = o1 - 2;
-        const int ci = cidx(d, 1 - g, k, l), co = cidx(d, d.nx + g, k, l);
-        d.P[1][ci] = dmin(d.P[1][ci], 0.0);
-        d.P[1][co] = dmax(d.P[1][co], 0.0);
-    }
-    if (d.bc_kind == 1 && o0 < d.NX && o1 < d.NY) {  // z ghosts: (j = o0-2, k = o1-2), not at cuts
-        const int j = o0 - 2, k = o1 - 2;
-        const int ci = cidx(d, j, k, 1 - g), co = cidx(d, j, k, d.nz + g);
-        if (d.zcut[0] != 1) d.P[3][ci] = dmin(d.P[3][ci], 0.0);
-        if (d.zcut[1] != 1) d.P[3][co] = dmax(d.P[3][co], 0.0);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// edge EMFs, mhd_module.f90:364-432
-// ---------------------------------------------------------------------------
-__global__ void k_edge(const Dev d) {
-    if (d.S->done) return;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = blockIdx.y * blockDim.y + threadIdx.y;
-    const int l = blockIdx.z;
-    if (j > d.nx || k > d.ny || l > d.nz) return;
+    // a z side shared with a neighbouring slab is filled by the exchange
+    if ((l < 1 && d.zcut[0]) || (l > d.nz && d.zcut[1])) return;
     const int c = cidx(d, j, k, l);
-    if (d.fix_n && (j | k | l) == 0) *d.fix_n = 0;  // k_faces_deferred has worked it off
-    const int sy = d.NX, sz = d.NX * d.NY;
+    int side[3], off[3];
     {
-        const double *fxy = d.EF[e_xy], *fxz = d.EF[e_xz], *ex = d.EC[0];
-        d.EX[c] = 0.50 * (fxy[c] + fxy[c + sz] + fxz[c] + fxz[c + sy])
-                  - 0.25 * (ex[c] + ex[c + sz] + ex[c + sy] + ex[c + sy + sz]);
+        const int i3[3] = {j, k, l}, n3[3] = {d.nx, d.ny, d.nz}, st[3] = {1, d.NX, d.NX * d.NY};
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+            side[x] = -1;
+            off[x] = 0;
+            if (i3[x] >= 1 && i3[x] <= n3[x]) continue;
+            const int s = i3[x] < 1 ? 0 : 1;
+            side[x] = 2 * x + s;
+            off[x] = (ghost_src(d.bf[side[x]], s == 0, s == 0 ? 1 - i3[x] : i3[x] - n3[x], n3[x]) - i3[x]) * st[x];
+        }
     }
-    {
-        const double *fyx = d.EF[e_yx], *fyz = d.EF[e_yz], *ey = d.EC[1];
-        d.EY[c] = 0.50 * (fyx[c] + fyx[c + sz] + fyz[c] + fyz[c + 1])
-                  - 0.25 * (ey[c] + ey[c + sz] + ey[c + 1] + ey[c + 1 + sz]);
+    const int first = blockIdx.y < 2 ? 4 * blockIdx.y : blockIdx.y == 2 ? 8 : 11;
+    const int last = blockIdx.y < 2 ? first + 4 : blockIdx.y == 2 ? 11 : 13;
+    double v[4];
+    bool moved[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int m = first + q;
+        v[q] = 0.0;
+        moved[q] = false;
+        if (m >= last) continue;
+        int o = 0;
+#pragma unroll
+        for (int x = 0; x < 3; ++x)
+            if (gl.axes[m] >> x & 1) o += off[x];
+        if (m == 12 && k > d.ny)  // epsilon: the BOUNDARY1D_NM y-outer rule (boundary.f90:243-282)
+            o += (d.eps_y_out_mode < 0 ? 0 : (ghost_src(d.eps_y_out_mode, false, k - d.ny, d.ny) - k) * d.NX) - off[1];
+        moved[q] = o != 0;
+        v[q] = gl.a[m][c + o];
+#pragma unroll
+        for (int x = 0; x < 3; ++x)
+            if ((gl.axes[m] >> x & 1) && side[x] >= 0 && d.bf[side[x]] >= 2)
+                v[q] = (double)d.bfac[side[x]][gl.var[m]] * v[q];
+        if (m == 1 && d.bc_kind != 0) {
+            if (j < 1) v[q] = dmin(v[q], 0.0);
+            if (j > d.nx) v[q] = dmax(v[q], 0.0);
+        }
+        if (m == 3 && d.bc_kind == 1) {
+            if (l < 1) v[q] = dmin(v[q], 0.0);
+            if (l > d.nz) v[q] = dmax(v[q], 0.0);
+        }
     }
-    {
-        const double *fzx = d.EF[e_zx], *fzy = d.EF[e_zy], *ez = d.EC[2];
-        d.EZ[c] = 0.50 * (fzx[c] + fzx[c + sy] + fzy[c] + fzy[c + 1])
-                  - 0.25 * (ez[c] + ez[c + sy] + ez[c + 1] + ez[c + 1 + sy]);
-    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        if (moved[q]) gl.a[first + q][c] = v[q];
 }
 
-// FIXPOLE, mhd_module.f90:437-461 (single-precision accumulators, sequential order)
-__global__ void k_fixpole(const Dev d) {
+// ---------------------------------------------------------------------------
+// edge EMFs, mhd_module.f90:364-432 with the 1D/2D face-EMF assignment (314-356)
+// and BOUNDARY_EFIELD (478-840) evaluated where an edge reads them: a ghost
+// value is a copy (times a parity) of an interior one, so an edge next to a
+// boundary maps its indices instead of reading a filled layer.  The cell EMFs
+// come from the recovery, which has their operands in registers.  (Forming them
+// here as well, from six arrays at seven cells, took 2.95 ms a 256^3 step: 48
+// loads an edge triple; 24 loads of which half hit L1 now.)
+// ---------------------------------------------------------------------------
+// PAR: some side has a parity rule.  Every lane takes the same path: the
+// offsets of an edge's cells and faces are computed per axis (unmoved inside the
+// grid), so the lanes at a boundary cost no divergence.
+template <int PAR>
+__global__ void __launch_bounds__(256) k_edge(const Dev d) {
     if (d.S->done) return;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    if (j > d.nx) return;
-    float sum1 = 0.0f, sum2 = 0.0f;
-    for (int l = 1; l <= d.nz; ++l) {
-        sum1 = (float)((double)sum1 + d.EX[cidx(d, j, 0, l)]);
-        sum2 = (float)((double)sum2 + d.EX[cidx(d, j, d.ny, l)]);
+    // flat index over j,k,l = 0..n (x fastest)
+    const unsigned ex = d.nx + 1, ey = d.ny + 1, ez = d.nz + 1;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= ex * ey * ez) return;
+    if (d.fix_n && t == 0) *d.fix_n = 0;  // k_faces_deferred has worked it off
+    int j, k, l;
+    unflat3(t, ex, ey, j, k, l);
+    const int c = cidx(d, j, k, l);
+    // per axis and step 0, 1: the offset of index i + step as BOUNDARY_EFIELD
+    // maps it (m), the same along a face's own axis (f: not mapped; a direction
+    // the grid does not have takes the cell EMF of its one cell on both faces),
+    // and the side whose parity applies
+    int m[3][2], f[3][2], side[3][2];
+    {
+        const int i3[3] = {j, k, l}, n3[3] = {d.nx, d.ny, d.nz}, st[3] = {1, d.NX, d.NX * d.NY};
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                const int i = i3[x] + s;
+                int src = i, sd = -1;
+                if (i < 1 && !(x == 2 && d.zcut[0])) {
+                    sd = 2 * x;
+                    src = d.bf[sd] == 0 ? n3[x] : 1;
+                } else if (i > n3[x] && !(x == 2 && d.zcut[1])) {
+                    sd = 2 * x + 1;
+                    src = d.bf[sd] == 0 ? 1 : n3[x];
+                }
+                m[x][s] = (src - i3[x]) * st[x];
+                f[x][s] = x < d.n_dim ? s * st[x] : (1 - i3[x]) * st[x];
+                side[x][s] = sd;
+            }
+        }
     }
-    const double a = (double)sum1 / (double)d.nz, b = (double)sum2 / (double)d.nz;
-    for (int l = -2; l <= d.nz + 3; ++l) {
-        d.EX[cidx(d, j, 0, l)] = a;
-        d.EX[cidx(d, j, d.ny, l)] = b;
+    // component q at steps (a, b, g) along x, y, z; own: the axis of the face
+    auto at = [&](const double *p, int q, int own, int a, int b, int g) {
+        const double v = p[c + (own == 0 ? f[0][a] : m[0][a]) + (own == 1 ? f[1][b] : m[1][b]) +
+                           (own == 2 ? f[2][g] : m[2][g])];
+        if (!PAR) return v;
+        double r = v;
+        const int sd[3] = {side[0][a], side[1][b], side[2][g]};
+#pragma unroll
+        for (int x = 0; x < 3; ++x)
+            if (x != own && sd[x] >= 0 && d.bf[sd[x]] >= 2) r = (double)d.bfac[sd[x]][9 + q] * r;  // iex = 9
+        return r;
+    };
+    const double *fxy = d.n_dim > 1 ? d.EF[e_xy] : d.EC[0], *fxz = d.n_dim > 2 ? d.EF[e_xz] : d.EC[0];
+    const double *fyx = d.EF[e_yx], *fyz = d.n_dim > 2 ? d.EF[e_yz] : d.EC[1];
+    const double *fzx = d.EF[e_zx], *fzy = d.n_dim > 1 ? d.EF[e_zy] : d.EC[2];
+    const double *cx = d.EC[0], *cy = d.EC[1], *cz = d.EC[2];
+    const double x = 0.50 * (at(fxy, 0, 1, 0, 0, 0) + at(fxy, 0, 1, 0, 0, 1) + at(fxz, 0, 2, 0, 0, 0) + at(fxz, 0, 2, 0, 1, 0))
+                     - 0.25 * (at(cx, 0, 3, 0, 0, 0) + at(cx, 0, 3, 0, 0, 1) + at(cx, 0, 3, 0, 1, 0) + at(cx, 0, 3, 0, 1, 1));
+    const double y = 0.50 * (at(fyx, 1, 0, 0, 0, 0) + at(fyx, 1, 0, 0, 0, 1) + at(fyz, 1, 2, 0, 0, 0) + at(fyz, 1, 2, 1, 0, 0))
+                     - 0.25 * (at(cy, 1, 3, 0, 0, 0) + at(cy, 1, 3, 0, 0, 1) + at(cy, 1, 3, 1, 0, 0) + at(cy, 1, 3, 1, 0, 1));
+    const double z = 0.50 * (at(fzx, 2, 0, 0, 0, 0) + at(fzx, 2, 0, 0, 1, 0) + at(fzy, 2, 1, 0, 0, 0) + at(fzy, 2, 1, 1, 0, 0))
+                     - 0.25 * (at(cz, 2, 3, 0, 0, 0) + at(cz, 2, 3, 0, 1, 0) + at(cz, 2, 3, 1, 0, 0) + at(cz, 2, 3, 1, 1, 0));
+    d.EX[c] = x;
+    d.EY[c] = y;
+    d.EZ[c] = z;
+}
+
+// FIXPOLE, mhd_module.f90:437-461 (single-precision accumulators, sequential
+// order).  A CTA takes 32 r cells: its eight warps bring 32 phi rows of both
+// poles into shared memory at a time, the first two add them up in order (the
+// sum is one chain of conversions and additions, nz long), then all write the
+// averages.  One thread per r cell that also loaded its terms one by one took
+// 140 us a stage at nz = 128, this 9.
+__global__ void __launch_bounds__(256) k_fixpole(const Dev d) {
+    if (d.S->done) return;
+    __shared__ double row[2][32][33];
+    __shared__ double mean[2][32];
+    const int tx = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int j = blockIdx.x * 32 + tx + 1;
+    const bool in = j <= d.nx;
+    float sum = 0.0f;
+    for (int l0 = 1; l0 <= d.nz; l0 += 32) {
+        for (int i = w; i < 64; i += 8) {
+            const int p = i >> 5, l = l0 + (i & 31);
+            if (in && l <= d.nz) row[p][i & 31][tx] = d.EX[cidx(d, j, p ? d.ny : 0, l)];
+        }
+        __syncthreads();
+        if (w < 2) {
+            const int m = d.nz - l0 + 1 < 32 ? d.nz - l0 + 1 : 32;
+#pragma unroll 8
+            for (int i = 0; i < m; ++i) sum = (float)((double)sum + row[w][i][tx]);
+        }
+        __syncthreads();
+    }
+    if (w < 2) mean[w][tx] = (double)sum / (double)d.nz;
+    __syncthreads();
+    if (!in) return;
+    for (int l = w - 2; l <= d.nz + 3; l += 8) {
+        d.EX[cidx(d, j, 0, l)] = mean[0][tx];
+        d.EX[cidx(d, j, d.ny, l)] = mean[1][tx];
     }
 }
 
@@ -624,6 +672,88 @@ __global__ void __launch_bounds__(256, 2) k_rk_cart(const Dev d, int stage) {
 }
 
 // ---------------------------------------------------------------------------
+// FINDDT, rungekutta.f90:221-332
+// ---------------------------------------------------------------------------
+// the CFL limit of one cell
+__device__ __forceinline__ double cell_dt(const Dev &d, int j, int k, int l, double rho, double vx, double vy, double vz,
+                                          double bx, double by, double bz, double cs) {
+    const double a2 = cs * cs;
+    const double a4 = a2 * a2;
+    double lambda, t = DX(j);
+    if (d.coord == 0) {
+        if (d.n_dim > 1) t = dmin(t, DY(k));
+        if (d.n_dim > 2) t = dmin(t, DZ(l));
+    } else if (d.coord == 1) {
+        if (d.n_dim > 1 && d.ny > 1) t = dmin(t, XC(j) * DY(k));
+        if (d.n_dim > 2) t = dmin(t, DZ(l));
+    } else {
+        if (d.n_dim > 1) t = dmin(t, XC(j) * DY(k));
+        if (d.n_dim > 2) t = dmin(t, XC(j) * SINE(k) * DZ(l));
+    }
+    t = t * d.cfl;
+    // branch-free where every operand is far from the ends of its range (a
+    // B^2 / rho too small to round right is lost beside a2)
+    {
+        const Den64 r = den64(rho);
+        const double b2x = quo(bx * bx, r.b, r.y), b2y = quo(by * by, r.b, r.y), b2z = quo(bz * bz, r.b, r.y);
+        const double b2 = b2x + b2y + b2z, b4 = b2 * b2, s = a4 + 2.0 * a2 * b2 + b4;
+        const double qx = s - 4.0 * a2 * b2x, qy = s - 4.0 * a2 * b2y, qz = s - 4.0 * a2 * b2z;
+        const double cfx = sqrt64(0.5 * (a2 + b2 + sqrt64(qx)));
+        const double cfy = sqrt64(0.5 * (a2 + b2 + sqrt64(qy)));
+        const double cfz = sqrt64(0.5 * (a2 + b2 + sqrt64(qz)));
+        lambda = dmax3(fabs(vx) + cfx, fabs(vy) + cfy, fabs(vz) + cfz);
+        const Den64 g = den64(lambda);
+        if (r.ok & g.ok & in_pos(a2, -120, 120) & in_pos(qx, -400, 400) & in_pos(qy, -400, 400) & in_pos(qz, -400, 400) &
+            in_pos(t, -200, 200))
+            return quo(t, g.b, g.y);
+    }
+    const double b2x = bx * bx / rho, b2y = by * by / rho, b2z = bz * bz / rho;
+    const double b2 = b2x + b2y + b2z;
+    const double b4 = b2 * b2;
+    const double cfx = sqrt(0.5 * (a2 + b2 + sqrt((a4 + 2.0 * a2 * b2 + b4) - 4.0 * a2 * b2x)));
+    const double cfy = sqrt(0.5 * (a2 + b2 + sqrt((a4 + 2.0 * a2 * b2 + b4) - 4.0 * a2 * b2y)));
+    const double cfz = sqrt(0.5 * (a2 + b2 + sqrt((a4 + 2.0 * a2 * b2 + b4) - 4.0 * a2 * b2z)));
+    lambda = dmax3(fabs(vx) + cfx, fabs(vy) + cfy, fabs(vz) + cfz);
+    return t / lambda;
+}
+
+// the block's minimum into dt_bits (every thread of the block calls it):
+// positive doubles order like their bit patterns, so the result is exact and
+// independent of order
+__device__ __forceinline__ void dt_min(const Dev &d, double dtt) {
+    unsigned long long bits = (unsigned long long)__double_as_longlong(dtt);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        unsigned long long o = __shfl_xor_sync(0xffffffffu, bits, off);
+        bits = o < bits ? o : bits;
+    }
+    __shared__ unsigned long long wmin[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) wmin[warp] = bits;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long b = wmin[0];
+        for (int w = 1; w < (int)blockDim.x >> 5; ++w) b = wmin[w] < b ? wmin[w] : b;
+        if (b < *(volatile unsigned long long *)&d.S->dt_bits) atomicMin(&d.S->dt_bits, b);
+    }
+}
+
+__global__ void __launch_bounds__(256) k_finddt(const Dev d) {
+    if (d.S->done) return;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    double dtt = 1.0e5;
+    if (t < (unsigned)d.nx * d.ny * d.nz) {
+        int j, k, l;
+        unflat3(t, d.nx, d.ny, j, k, l);
+        const int c = cidx(d, j + 1, k + 1, l + 1);
+        const double lim = cell_dt(d, j + 1, k + 1, l + 1, d.P[0][c], d.P[1][c], d.P[2][c], d.P[3][c], d.BC[0][c],
+                                   d.BC[1][c], d.BC[2][c], d.CS[c]);
+        if (lim < dtt) dtt = lim;  // NaN never wins (the oracle's comparison)
+    }
+    dt_min(d, dtt);
+}
+
+// ---------------------------------------------------------------------------
 // recovery on the interior: FROMUTORVE (fromrvetou.f90:126-227), the model
 // floors (CUSTOM_CHECKRHO), FROMRVETOU (21-121) and FINDPRESSURE.
 // INIT = 1 is INITIAL_UPDATE's CHECKRHO -> FROMRVETOU -> FINDPRESSURE.
@@ -674,8 +804,9 @@ __device__ __forceinline__ void apply_floor(const Dev &d, double &rho, double &v
 // u_c the hydro part, bfx..bfz its own new face fields, ux_m..uz_m the new
 // fields of its lower faces; px_m..pz_m the lower faces' primitive fields
 // (used on the index-1 layers, whose lower face FROMUTORVE leaves alone).
-template <int INIT>
-__device__ __forceinline__ void recover_cell(const Dev &d, int stage, int j, int k, int l, int c, const double *u_c,
+// DT: returns the cell's CFL limit.
+template <int INIT, int DT>
+__device__ __forceinline__ double recover_cell(const Dev &d, int stage, int j, int k, int l, int c, const double *u_c,
                                              double bfx, double bfy, double bfz, double ux_m, double uy_m,
                                              double uz_m, double px_m, double py_m, double pz_m) {
     double rho, vx, vy, vz, e, bc[3];
@@ -771,124 +902,72 @@ __device__ __forceinline__ void recover_cell(const Dev &d, int stage, int j, int
     d.BC[1][c] = bc[1];
     d.BC[2][c] = bc[2];
     d.CS[c] = cs;
+    // the cell EMF -v x B of the next stage (mhd_module.f90:310-312)
+    d.EC[0][c] = vz * bc[1] - vy * bc[2];
+    d.EC[1][c] = vx * bc[2] - vz * bc[0];
+    d.EC[2][c] = vy * bc[0] - vx * bc[1];
     // guard: a state no later stage can recover from
     if (!(rho > 0.0) || !isfinite(e) || !isfinite(p) || !isfinite(vx) || !isfinite(vy) || !isfinite(vz) || !isfinite(cs))
         set_error(d, CUMC_ESTATE, c, stage);
+    return DT ? cell_dt(d, j, k, l, rho, vx, vy, vz, bc[0], bc[1], bc[2], cs) : 0.0;
 }
 
-template <int INIT>
-__global__ void __launch_bounds__(256) k_recover(const Dev d, int stage) {
-    if (d.S->done) return;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int k = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    const int l = blockIdx.z + 1;
-    if (j > d.nx || k > d.ny || l > d.nz) return;
-    const int c = cidx(d, j, k, l);
-    const int sy = d.NX, sz = d.NX * d.NY;
-    double bfx = 0.0, bfy = 0.0, bfz = 0.0;
-    // every load of the cell issued before any arithmetic (the kernel waits on
-    // memory, not on its few flops); the lower-face operands of FROMRVETOU are
-    // selected afterwards from loads of both candidates
-    double ux_m = 0.0, uy_m = 0.0, uz_m = 0.0, u_c[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    const double px_m = d.P[5][c - 1], py_m = d.P[6][c - sy], pz_m = d.P[7][c - sz];
-    if (!INIT) {
-        bfx = d.U[5][c]; bfy = d.U[6][c]; bfz = d.U[7][c];
-        ux_m = d.U[5][c - 1]; uy_m = d.U[6][c - sy]; uz_m = d.U[7][c - sz];
-#pragma unroll
-        for (int i = 0; i < 5; ++i) u_c[i] = d.U[i][c];
-    }
-    recover_cell<INIT>(d, stage, j, k, l, c, u_c, bfx, bfy, bfz, ux_m, uy_m, uz_m, px_m, py_m, pz_m);
-}
-
-// FROMRVETOU on the index-0 layer: cons face fields = prim face fields.  A
+// FROMRVETOU on the index-0 layer: cons face fields = prim face fields (before
+// the ghost fill).  The cells next to the layer carry it: cell (j, k, l) the
+// index-0 cells below it, (1, k, l) also after its own read of their faces.  A
 // slab's lower cut plane interior to the whole grid (zcut 1) takes the prim
 // values once (INITIAL_UPDATE, as every interior cell), then evolves by
 // constrained transport; the seam of a periodic ring (zcut 2) is the whole
 // grid's boundary and keeps the rule.
-__global__ void k_cons0(const Dev d, int init) {
-    if (d.S->done) return;
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    const int b = blockIdx.y;
-    const int plane = blockIdx.z;
-    int j, k, l;
-    if (plane == 0) { if (a > d.ny || b > d.nz) return; j = 0; k = a; l = b; }
-    else if (plane == 1) { if (a > d.nx || b > d.nz) return; j = a; k = 0; l = b; }
-    else { if (a > d.nx || b > d.ny || (d.zcut[0] == 1 && !init)) return; j = a; k = b; l = 0; }
-    const int c = cidx(d, j, k, l);
-    d.U[5][c] = d.P[5][c];
-    d.U[6][c] = d.P[6][c];
-    d.U[7][c] = d.P[7][c];
+__device__ __forceinline__ void cons_layer0(const Dev &d, int init, int j, int k, int l, int c) {
+    const int sy = d.NX, sz = d.NX * d.NY;
+#pragma unroll 1
+    for (int m = 1; m < 8; ++m) {
+        if (((m & 1) && j > 1) || ((m & 2) && k > 1) || ((m & 4) && l > 1)) continue;
+        if (m == 4 && d.zcut[0] == 1 && !init) continue;
+        const int q = c - (m & 1) - ((m >> 1) & 1) * sy - (m >> 2) * sz;
+        for (int v = 5; v < 8; ++v) d.U[v][q] = d.P[v][q];
+    }
 }
 
-// ---------------------------------------------------------------------------
-// FINDDT, rungekutta.f90:221-332
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_finddt(const Dev d) {
+// INIT: INITIAL_UPDATE's pass.  DT: also reduce FINDDT's minimum, on the values
+// at hand (the last stage inside cumc_evolve; a pass of its own over eight
+// arrays took 0.32 ms of a 256^3 step).
+template <int INIT, int DT>
+__global__ void __launch_bounds__(256) k_recover(const Dev d, int stage) {
     if (d.S->done) return;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int k = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    const int l = blockIdx.z + 1;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     double dtt = 1.0e5;
-    if (j <= d.nx && k <= d.ny && l <= d.nz) {
+    if (t < (unsigned)d.nx * d.ny * d.nz) {
+        int j, k, l;
+        unflat3(t, d.nx, d.ny, j, k, l);
+        ++j;
+        ++k;
+        ++l;
         const int c = cidx(d, j, k, l);
-        const double rho = d.P[0][c];
-        const double a2 = d.CS[c] * d.CS[c];
-        const double a4 = a2 * a2;
-        const double bx = d.BC[0][c], by = d.BC[1][c], bz = d.BC[2][c];
-        const double b2x = dv(bx * bx, rho);
-        const double b2y = dv(by * by, rho);
-        const double b2z = dv(bz * bz, rho);
-        const double b2 = b2x + b2y + b2z;
-        const double b4 = b2 * b2;
-        const double cfx = sqrt(0.5 * (a2 + b2 + sqrt((a4 + 2.0 * a2 * b2 + b4) - 4.0 * a2 * b2x)));
-        const double cfy = sqrt(0.5 * (a2 + b2 + sqrt((a4 + 2.0 * a2 * b2 + b4) - 4.0 * a2 * b2y)));
-        const double cfz = sqrt(0.5 * (a2 + b2 + sqrt((a4 + 2.0 * a2 * b2 + b4) - 4.0 * a2 * b2z)));
-        const double lambda1 = fabs(d.P[1][c]) + cfx;
-        const double lambda2 = fabs(d.P[2][c]) + cfy;
-        const double lambda3 = fabs(d.P[3][c]) + cfz;
-        const double lambda = dmax3(lambda1, lambda2, lambda3);
-        double t = DX(j);
-        if (d.coord == 0) {
-            if (d.n_dim > 1) t = dmin(t, DY(k));
-            if (d.n_dim > 2) t = dmin(t, DZ(l));
-        } else if (d.coord == 1) {
-            if (d.n_dim > 1 && d.ny > 1) t = dmin(t, XC(j) * DY(k));
-            if (d.n_dim > 2) t = dmin(t, DZ(l));
-        } else {
-            if (d.n_dim > 1) t = dmin(t, XC(j) * DY(k));
-            if (d.n_dim > 2) t = dmin(t, XC(j) * SINE(k) * DZ(l));
-        }
-        t = t * d.cfl / lambda;
-        if (t < dtt) dtt = t;  // NaN never wins (the oracle's comparison)
-    }
-    // deterministic min: positive doubles order like their bit patterns
-    unsigned long long bits = (unsigned long long)__double_as_longlong(dtt);
+        const int sy = d.NX, sz = d.NX * d.NY;
+        double bfx = 0.0, bfy = 0.0, bfz = 0.0;
+        // every load of the cell issued before any arithmetic (the kernel waits
+        // on memory, not on its few flops); the lower-face operands of FROMRVETOU
+        // are selected afterwards from loads of both candidates
+        double ux_m = 0.0, uy_m = 0.0, uz_m = 0.0, u_c[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        const double px_m = d.P[5][c - 1], py_m = d.P[6][c - sy], pz_m = d.P[7][c - sz];
+        if (!INIT) {
+            bfx = d.U[5][c]; bfy = d.U[6][c]; bfz = d.U[7][c];
+            ux_m = d.U[5][c - 1]; uy_m = d.U[6][c - sy]; uz_m = d.U[7][c - sz];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        unsigned long long o = __shfl_xor_sync(0xffffffffu, bits, off);
-        bits = o < bits ? o : bits;
-    }
-    __shared__ unsigned long long wmin[32];
-    const int lane = (threadIdx.y * blockDim.x + threadIdx.x) & 31;
-    const int warp = (threadIdx.y * blockDim.x + threadIdx.x) >> 5;
-    if (lane == 0) wmin[warp] = bits;
-    __syncthreads();
-    if (warp == 0) {
-        const int nw = (blockDim.x * blockDim.y + 31) >> 5;
-        unsigned long long b = lane < nw ? wmin[lane] : ~0ull;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            unsigned long long o = __shfl_xor_sync(0xffffffffu, b, off);
-            b = o < b ? o : b;
+            for (int i = 0; i < 5; ++i) u_c[i] = d.U[i][c];
         }
-        if (lane == 0) atomicMin(&d.S->dt_bits, b);
+        const double lim =
+            recover_cell<INIT, DT>(d, stage, j, k, l, c, u_c, bfx, bfy, bfz, ux_m, uy_m, uz_m, px_m, py_m, pz_m);
+        if (DT && lim < dtt) dtt = lim;  // NaN never wins (the oracle's comparison)
+        if (j == 1 || k == 1 || l == 1) cons_layer0(d, INIT, j, k, l, c);
     }
+    if (DT) dt_min(d, dtt);
 }
 
 // dt = MIN(1.0D5, reduced); clamp to total_time (main.f90:104-106) when asked
-__global__ void k_dt_final(const Dev d, int clamp) {
-    if (d.S->done) return;
-    Scalars *S = d.S;
+__device__ __forceinline__ void dt_final(Scalars *S, int clamp) {
     double dt = __longlong_as_double((long long)S->dt_bits);
     if (!(dt < 1.0e5)) dt = 1.0e5;
     if (clamp && S->t + dt > S->t_end) dt = S->t_end - S->t;
@@ -896,16 +975,23 @@ __global__ void k_dt_final(const Dev d, int clamp) {
         if (S->err_code == 0) { S->err_code = CUMC_ESTATE; S->err_cell = -1; S->err_stage = 0; }
     }
     S->dt = dt;
-    S->dt_bits = (unsigned long long)__double_as_longlong(1.0e5);
+}
+__global__ void k_dt_final(const Dev d, int clamp) {
+    if (d.S->done) return;
+    dt_final(d.S, clamp);
+    d.S->dt_bits = (unsigned long long)__double_as_longlong(1.0e5);
 }
 
-// end of a step inside cumc_evolve: t += dt, count, stop conditions
-__global__ void k_step_end(const Dev d) {
+// the turn of a step inside cumc_evolve: t += dt, count, stop conditions, then
+// the next step's dt from the minimum the last stage reduced
+__global__ void k_step_turn(const Dev d) {
     Scalars *S = d.S;
     if (S->done) return;
     S->t = S->t + S->dt;
     S->steps += 1;
     if (!(S->t < S->t_end) || S->steps >= S->max_steps || S->err_code != 0) S->done = 1;
+    else dt_final(S, 1);
+    S->dt_bits = (unsigned long long)__double_as_longlong(1.0e5);
 }
 
 // FIND_DIVB, mhd_module.f90:110-201 (max |div B| from the face fields)
@@ -1325,72 +1411,24 @@ static void launch_flux(cumc_handle *h, int dir, int stage = 1, cudaStream_t st 
     h->launches++;
 }
 
-static FillList make_list(cumc_handle *h, int axis, int side) {
-    // side: 0 inner, 1 outer.  parity side index: 2*axis + side
+static void launch_ghosts(cumc_handle *h) {
     const Dev &d = h->d;
-    const signed char *bf = d.bfac[2 * axis + side];
-    FillList L;
-    L.n = 0;
-    auto add = [&](double *a, int var) { L.a[L.n] = a; L.par[L.n] = bf[var]; L.n++; };
-    for (int i = 0; i < 5; ++i) add(d.P[i], 1 + i);
-    for (int i = 0; i < 3; ++i) add(d.BC[i], 6 + i);
-    // transverse face fields of this axis (boundary.f90:432-433, 543-544, 654-655)
-    for (int i = 0; i < 3; ++i)
-        if (i != axis) add(d.P[5 + i], 6 + i);
-    if (d.fixn && d.bf[2 * axis] == 0) add(d.P[5 + axis], 6 + axis);
-    add(d.CS, 1);   // FINDPRESSURE output, even (recomputed identically by the reference)
-    if (axis != 1 || side == 0) add(d.EPS, 1);  // epsilon y-outer handled separately
-    return L;
-}
-
-static FillList make_elist(cumc_handle *h, int axis, int side) {
-    const Dev &d = h->d;
-    const signed char *bf = d.bfac[2 * axis + side];
-    enum { iex = 9, iey = 10, iez = 11 };
-    FillList L;
-    L.n = 0;
-    auto add = [&](double *a, int var) { L.a[L.n] = a; L.par[L.n] = bf[var]; L.n++; };
-    for (int i = 0; i < 3; ++i) add(d.EC[i], iex + i);
-    if (axis == 0) { add(d.EF[e_xz], iex); add(d.EF[e_xy], iex); add(d.EF[e_yz], iey); add(d.EF[e_zy], iez); }
-    else if (axis == 1) { add(d.EF[e_xz], iex); add(d.EF[e_yx], iey); add(d.EF[e_yz], iey); add(d.EF[e_zx], iez); }
-    else { add(d.EF[e_xy], iex); add(d.EF[e_yx], iey); add(d.EF[e_zx], iez); add(d.EF[e_zy], iez); }
-    return L;
-}
-
-static void launch_fills(cumc_handle *h, bool emf) {
-    const Dev &d = h->d;
-    for (int axis = 0; axis < 3; ++axis) {
-        FillList in = emf ? make_elist(h, axis, 0) : make_list(h, axis, 0);
-        FillList out = emf ? make_elist(h, axis, 1) : make_list(h, axis, 1);
-        // a z side shared with a neighbouring slab is filled by the exchange
-        if (axis == 2 && d.zcut[0]) in.n = 0;
-        if (axis == 2 && d.zcut[1]) out.n = 0;
-        int o0 = (axis == 0) ? d.NY : d.NX;
-        int o1 = (axis == 2) ? d.NY : d.NZ;
-        dim3 b(o0 >= 128 ? 128 : 32), g((o0 + b.x - 1) / b.x, o1, 3);
-        int mode = -1;
-        if (!emf && axis == 1) mode = d.eps_y_out_mode;
-        if (axis == 0) k_fill<0><<<g, b, 0, h->stream>>>(d, in, out, mode);
-        else if (axis == 1) k_fill<1><<<g, b, 0, h->stream>>>(d, in, out, mode);
-        else k_fill<2><<<g, b, 0, h->stream>>>(d, in, out, mode);
-        h->launches++;
-    }
-    if (!emf && d.bc_kind != 0) {
-        int o0 = d.NX > d.NY ? d.NX : d.NY;
-        int o1 = d.NY > d.NZ ? d.NY : d.NZ;
-        dim3 b(32), g((o0 + 31) / 32, o1, 3);
-        k_custom_bc<<<g, b, 0, h->stream>>>(d);
-        h->launches++;
-    }
-}
-
-static void launch_cons0(cumc_handle *h, int init = 0) {
-    const Dev &d = h->d;
-    int m = d.nx + 1;
-    if (d.ny + 1 > m) m = d.ny + 1;
-    int mb = (d.ny + 1 > d.nz + 1) ? d.ny + 1 : d.nz + 1;
-    dim3 b(32), g((m + 31) / 32, mb, 3);
-    k_cons0<<<g, b, 0, h->stream>>>(d, init);
+    GhostList g;
+    int n = 0;
+    auto add = [&](double *a, int var, int axes) {
+        g.a[n] = a;
+        g.var[n] = (unsigned char)var;
+        g.axes[n++] = (unsigned char)axes;
+    };
+    for (int i = 0; i < 5; ++i) add(d.P[i], 1 + i, 7);
+    for (int i = 0; i < 3; ++i) add(d.BC[i], 6 + i, 7);
+    // a face field: the transverse axes (boundary.f90:432-433, 543-544,
+    // 654-655), its own where the periodic-face option refills it
+    for (int i = 0; i < 3; ++i) add(d.P[5 + i], 6 + i, d.fixn && d.bf[2 * i] == 0 ? 7 : 7 & ~(1 << i));
+    add(d.CS, 1, 7);  // FINDPRESSURE output, even (recomputed identically by the reference)
+    add(d.EPS, 1, 7);
+    const long long cells = 6LL * d.NY * d.NZ + 6LL * d.nx * d.NZ + 6LL * d.nx * d.ny;
+    k_ghosts<<<dim3((unsigned)((cells + 255) / 256), GHOST_GROUPS), 256, 0, h->stream>>>(d, g);
     h->launches++;
 }
 
@@ -1409,18 +1447,18 @@ static void prof_end(cumc_handle *h, int cls) {
     h->prof_ms[cls] += ms;
 }
 
-// one RK stage (rungekutta.f90:61-100), in two halves: the face fluxes and
-// the cell EMFs with their ghosts (a), then the edge EMFs, the update, the
+// one RK stage (rungekutta.f90:61-100), in two halves: the face fluxes
+// (a), then the edge EMFs, the update, the
 // recovery and the state ghosts (b); a slab group exchanges ghost planes
 // after each half
 static void enqueue_stage_a(cumc_handle *h, int stage);
-static void enqueue_stage_b(cumc_handle *h, int stage);
-static void enqueue_stage(cumc_handle *h, int stage) {
+static void enqueue_stage_b(cumc_handle *h, int stage, bool with_dt = false);
+static void enqueue_stage(cumc_handle *h, int stage, bool with_dt = false) {
     enqueue_stage_a(h, stage);
-    enqueue_stage_b(h, stage);
+    enqueue_stage_b(h, stage, with_dt);
 }
 static void enqueue_stage_a(cumc_handle *h, int stage) {
-    Range r("cumc stage: face fluxes + cell EMFs");
+    Range r("cumc stage: face fluxes");
     const Dev &d = h->d;
     if (h->sweeps_concurrent && h->prof_class < 0 && !d.learned && d.n_dim > 1) {
         // fork: the sweeps after the previous stage's last kernel; join: the
@@ -1439,17 +1477,12 @@ static void enqueue_stage_a(cumc_handle *h, int stage) {
             prof_end(h, PC_FLUX_X + dir);
         }
     }
-    dim3 g, b;
-    prof_begin(h);
     if (d.fix_n) {
+        prof_begin(h);
         launch_faces_deferred(d, h->stream);
         h->launches++;
+        prof_end(h, PC_EMF);
     }
-    grid_dims(d, g, b, 1, d.nx, 1, d.ny, 1, d.nz);
-    k_ecell<<<g, b, 0, h->stream>>>(d);
-    h->launches++;
-    launch_fills(h, true);
-    prof_end(h, PC_EMF);
 }
 template <class FT>
 static void launch_rk(const Dev &d, int stage, long long cells, cudaStream_t s) {
@@ -1458,16 +1491,21 @@ static void launch_rk(const Dev &d, int stage, long long cells, cudaStream_t s) 
     else if (d.coord == 1) k_rk<FT, 1><<<g, 128, 0, s>>>(d, stage);
     else k_rk<FT, 2><<<g, 128, 0, s>>>(d, stage);
 }
-static void enqueue_stage_b(cumc_handle *h, int stage) {
+static unsigned cell_blocks(const Dev &d) { return (unsigned)(((long long)d.nx * d.ny * d.nz + 255) / 256); }
+static void enqueue_stage_b(cumc_handle *h, int stage, bool with_dt) {
     Range r("cumc stage: edge EMFs + update + recovery + ghosts");
     const Dev &d = h->d;
-    dim3 g, b;
     prof_begin(h);
-    grid_dims(d, g, b, 0, d.nx, 0, d.ny, 0, d.nz);
-    k_edge<<<g, b, 0, h->stream>>>(d);
+    {
+        const unsigned g = (unsigned)(((long long)(d.nx + 1) * (d.ny + 1) * (d.nz + 1) + 255) / 256);
+        bool par = false;
+        for (int i = 0; i < 6; ++i) par = par || d.bf[i] >= 2;
+        if (par) k_edge<1><<<g, 256, 0, h->stream>>>(d);
+        else k_edge<0><<<g, 256, 0, h->stream>>>(d);
+    }
     h->launches++;
     if (h->cfg.fixpole && d.coord == 2) {
-        k_fixpole<<<(d.nx + 127) / 128, 128, 0, h->stream>>>(d);
+        k_fixpole<<<(d.nx + 31) / 32, 256, 0, h->stream>>>(d);
         h->launches++;
     }
     prof_end(h, PC_EMF);
@@ -1486,13 +1524,12 @@ static void enqueue_stage_b(cumc_handle *h, int stage) {
     h->launches++;
     prof_end(h, PC_RK);
     prof_begin(h);
-    grid_dims(d, g, b, 1, d.nx, 1, d.ny, 1, d.nz);
-    k_recover<0><<<g, b, 0, h->stream>>>(d, stage);
+    if (with_dt) k_recover<0, 1><<<cell_blocks(d), 256, 0, h->stream>>>(d, stage);
+    else k_recover<0, 0><<<cell_blocks(d), 256, 0, h->stream>>>(d, stage);
     h->launches++;
-    launch_cons0(h);
     prof_end(h, PC_RECOVER);
     prof_begin(h);
-    launch_fills(h, false);
+    launch_ghosts(h);
     prof_end(h, PC_BND);
     if (d.source_kind == 4) {
         if (h->cfg.precision == CUMC_FP32) k_bh_update<float><<<1, 1024, 0, h->stream>>>(d, stage);
@@ -1503,20 +1540,19 @@ static void enqueue_stage_b(cumc_handle *h, int stage) {
 
 static void enqueue_finddt(cumc_handle *h, int clamp) {
     const Dev &d = h->d;
-    dim3 g, b;
     prof_begin(h);
-    grid_dims(d, g, b, 1, d.nx, 1, d.ny, 1, d.nz);
-    k_finddt<<<g, b, 0, h->stream>>>(d);
+    k_finddt<<<cell_blocks(d), 256, 0, h->stream>>>(d);
     k_dt_final<<<1, 1, 0, h->stream>>>(d, clamp);
     h->launches += 2;
     prof_end(h, PC_DT);
 }
 
-static void enqueue_step(cumc_handle *h, bool with_dt, bool end) {
-    if (with_dt) enqueue_finddt(h, 1);
-    for (int s = 1; s <= 3; ++s) enqueue_stage(h, s);
-    if (end) {
-        k_step_end<<<1, 1, 0, h->stream>>>(h->d);
+// the three stages of a step with dt on the device; turn: as cumc_evolve's
+// graph, which ends with the next step's dt
+static void enqueue_step(cumc_handle *h, bool turn) {
+    for (int s = 1; s <= 3; ++s) enqueue_stage(h, s, turn && s == 3);
+    if (turn) {
+        k_step_turn<<<1, 1, 0, h->stream>>>(h->d);
         h->launches++;
     }
 }
@@ -1870,12 +1906,9 @@ int cumc_get_array(cumc_handle *h, int which, double *out, size_t n_doubles) {
 // INITIAL_UPDATE (initial.f90:86-116): CHECKRHO, FROMRVETOU, BOUNDARY, UPDATE
 static void enqueue_initial(cumc_handle *h) {
     const Dev &d = h->d;
-    dim3 g, b;
-    grid_dims(d, g, b, 1, d.nx, 1, d.ny, 1, d.nz);
-    k_recover<1><<<g, b, 0, h->stream>>>(d, 0);
+    k_recover<1, 0><<<cell_blocks(d), 256, 0, h->stream>>>(d, 0);
     h->launches++;
-    launch_cons0(h, 1);
-    launch_fills(h, false);
+    launch_ghosts(h);
 }
 
 int cumc_initial_update(cumc_handle *h) {
@@ -1910,7 +1943,7 @@ int cumc_rk3_step(cumc_handle *h, double dt) {
     if (h->d.source_kind == CUMC_SRC_COLLAPSAR && !h->d.phi[0])
         return fail(h, CUMC_ENOTREADY, "the collapsar source needs cumc_poisson_setup first");
     CK(cudaMemcpyAsync(&h->d.S->dt, &dt, sizeof(double), cudaMemcpyHostToDevice, h->stream));
-    enqueue_step(h, false, false);
+    enqueue_step(h, false);
     CK(cudaGetLastError());
     return check_scalars(h);
 }
@@ -1933,18 +1966,20 @@ int cumc_evolve(cumc_handle *h, double t_end, int max_steps, double *t_inout, in
     s.steps = 0;
     s.max_steps = max_steps;
     s.done = 0;
+    s.dt_bits = (unsigned long long)0x40F86A0000000000ull;  // bits of 1.0e5
     *h->S_host = s;
     CK(cudaMemcpyAsync(h->d.S, h->S_host, sizeof(Scalars), cudaMemcpyHostToDevice, h->stream));
     // capture one step the first time
     if (!h->graph_exec) {
         int64_t before = h->launches;
         CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        enqueue_step(h, true, true);
+        enqueue_step(h, true);
         CK(cudaStreamEndCapture(h->stream, &h->graph));
         CK(cudaGraphInstantiate(&h->graph_exec, h->graph, 0));
         h->kernels_per_step = (int)(h->launches - before);
         h->launches = before;
     }
+    enqueue_finddt(h, 1);  // the first step's dt; each step's turn makes the next
     // replay in chunks; kernels turn into no-ops once the device sets done
     int issued = 0;
     while (true) {
