@@ -95,6 +95,7 @@ constexpr int GHOST_GROUPS = 4;  // blockIdx.y: arrays 0-3, 4-7, 8-10, 11-12
 // No source is itself written: on every axis that moves it is an interior index.
 // Three dependent passes and the clamps took four launches a stage.
 __global__ void __launch_bounds__(256) k_ghosts(const Dev d, const GhostList gl) {
+    pdl_wait();
     if (d.S->done) return;
     unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     // cells with a ghost index in x, then in y, then in z only
@@ -188,6 +189,7 @@ __global__ void __launch_bounds__(256) k_ghosts(const Dev d, const GhostList gl)
 // grid), so the lanes at a boundary cost no divergence.
 template <int PAR>
 __global__ void __launch_bounds__(256) k_edge(const Dev d) {
+    pdl_wait();
     if (d.S->done) return;
     // flat index over j,k,l = 0..n (x fastest)
     const unsigned ex = d.nx + 1, ey = d.ny + 1, ez = d.nz + 1;
@@ -257,6 +259,7 @@ __global__ void __launch_bounds__(256) k_edge(const Dev d) {
 // averages.  One thread per r cell that also loaded its terms one by one took
 // 140 us a stage at nz = 128, this 9.
 __global__ void __launch_bounds__(256) k_fixpole(const Dev d) {
+    pdl_wait();
     if (d.S->done) return;
     __shared__ double row[2][32][33];
     __shared__ double mean[2][32];
@@ -296,6 +299,7 @@ __global__ void __launch_bounds__(256) k_fixpole(const Dev d) {
 // ---------------------------------------------------------------------------
 template <class FT>
 __global__ void __launch_bounds__(1024) k_bh_update(const Dev d, int stage) {
+    pdl_wait();
     if (d.S->done) return;
     __shared__ double part[1024];
     const int t = threadIdx.x;
@@ -577,6 +581,7 @@ __device__ __forceinline__ void rk_cell(const Dev &d, int stage, int j, int k, i
 
 template <class FT, int COORD>  // storage type of the hydro face fluxes (double, or float in the FP32 form)
 __global__ void __launch_bounds__(128, 3) k_rk(const Dev d, int stage) {
+    pdl_wait();
     if (d.S->done) return;
     // flat index over j,k,l = 0..n (x fastest)
     // (64-bit index arithmetic: the 32-bit form, cheaper in instructions,
@@ -603,6 +608,7 @@ __global__ void __launch_bounds__(128, 3) k_rk(const Dev d, int stage) {
 // bits.  (For the FP64 form the hoisted FP64 fluxes spill; k_rk stays.)
 template <class FT>
 __global__ void __launch_bounds__(256, 2) k_rk_cart(const Dev d, int stage) {
+    pdl_wait();
     if (d.S->done) return;
     const unsigned ex = d.nx + 1, ey = d.ny + 1, ez = d.nz + 1;
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -739,6 +745,7 @@ __device__ __forceinline__ void dt_min(const Dev &d, double dtt) {
 }
 
 __global__ void __launch_bounds__(256) k_finddt(const Dev d) {
+    pdl_wait();
     if (d.S->done) return;
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     double dtt = 1.0e5;
@@ -935,6 +942,7 @@ __device__ __forceinline__ void cons_layer0(const Dev &d, int init, int j, int k
 // arrays took 0.32 ms of a 256^3 step).
 template <int INIT, int DT>
 __global__ void __launch_bounds__(256) k_recover(const Dev d, int stage) {
+    pdl_wait();
     if (d.S->done) return;
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     double dtt = 1.0e5;
@@ -977,6 +985,7 @@ __device__ __forceinline__ void dt_final(Scalars *S, int clamp) {
     S->dt = dt;
 }
 __global__ void k_dt_final(const Dev d, int clamp) {
+    pdl_wait();
     if (d.S->done) return;
     dt_final(d.S, clamp);
     d.S->dt_bits = (unsigned long long)__double_as_longlong(1.0e5);
@@ -985,6 +994,7 @@ __global__ void k_dt_final(const Dev d, int clamp) {
 // the turn of a step inside cumc_evolve: t += dt, count, stop conditions, then
 // the next step's dt from the minimum the last stage reduced
 __global__ void k_step_turn(const Dev d) {
+    pdl_wait();
     Scalars *S = d.S;
     if (S->done) return;
     S->t = S->t + S->dt;
@@ -1145,7 +1155,7 @@ struct cumc_handle {
     bool have_state = false;
     bool initialised = false;
     int64_t launches = 0;
-    int kernels_per_step = 0;
+    int kernels_per_step[2] = {0, 0};
     // flux tiles (autotuned or default): block dims per direction
     dim3 fblk[3];
     int flux_mode = 1;  // 0 fused recon+Riemann kernel, 1 split kernels
@@ -1156,9 +1166,11 @@ struct cumc_handle {
     cudaStream_t fstream[2] = {nullptr, nullptr};
     cudaEvent_t fev[3] = {nullptr, nullptr, nullptr};
     void *qsets[2][14] = {};   // QL[0..6], QR[0..6] of sweeps 1 and 2
-    // captured step graph
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t graph_exec = nullptr;
+    // captured steps: [0] cumc_evolve's (ends with the next dt), [1] the three
+    // stages alone (cumc_rk3_step, from its third call on)
+    cudaGraph_t graph[2] = {nullptr, nullptr};
+    cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};
+    int eager_steps = 0;
     Scalars *S_host = nullptr;  // pinned mirror
     unsigned long long *divb_dev = nullptr;
     double *stage_aos = nullptr;   // 8*N3 doubles (the u_old block doubles as transpose staging)
@@ -1428,8 +1440,19 @@ static void launch_ghosts(cumc_handle *h) {
     add(d.CS, 1, 7);  // FINDPRESSURE output, even (recomputed identically by the reference)
     add(d.EPS, 1, 7);
     const long long cells = 6LL * d.NY * d.NZ + 6LL * d.nx * d.NZ + 6LL * d.nx * d.ny;
-    k_ghosts<<<dim3((unsigned)((cells + 255) / 256), GHOST_GROUPS), 256, 0, h->stream>>>(d, g);
+    launch(k_ghosts, dim3((unsigned)((cells + 255) / 256), GHOST_GROUPS), 256, 0, h->stream, d.pdl, d, g);
     h->launches++;
+}
+
+// the captured steps hold the kernels' parameters and launch shapes
+static void drop_graphs(cumc_handle *h) {
+    for (int i = 0; i < 2; ++i) {
+        if (h->graph_exec[i]) cudaGraphExecDestroy(h->graph_exec[i]);
+        if (h->graph[i]) cudaGraphDestroy(h->graph[i]);
+        h->graph_exec[i] = nullptr;
+        h->graph[i] = nullptr;
+    }
+    h->eager_steps = 0;
 }
 
 // kernel classes timed by cumc_profile_step
@@ -1487,9 +1510,9 @@ static void enqueue_stage_a(cumc_handle *h, int stage) {
 template <class FT>
 static void launch_rk(const Dev &d, int stage, long long cells, cudaStream_t s) {
     const unsigned g = (unsigned)((cells + 127) / 128);
-    if (d.coord == 0) k_rk<FT, 0><<<g, 128, 0, s>>>(d, stage);
-    else if (d.coord == 1) k_rk<FT, 1><<<g, 128, 0, s>>>(d, stage);
-    else k_rk<FT, 2><<<g, 128, 0, s>>>(d, stage);
+    if (d.coord == 0) launch(k_rk<FT, 0>, g, 128, 0, s, d.pdl, d, stage);
+    else if (d.coord == 1) launch(k_rk<FT, 1>, g, 128, 0, s, d.pdl, d, stage);
+    else launch(k_rk<FT, 2>, g, 128, 0, s, d.pdl, d, stage);
 }
 static unsigned cell_blocks(const Dev &d) { return (unsigned)(((long long)d.nx * d.ny * d.nz + 255) / 256); }
 static void enqueue_stage_b(cumc_handle *h, int stage, bool with_dt) {
@@ -1500,12 +1523,12 @@ static void enqueue_stage_b(cumc_handle *h, int stage, bool with_dt) {
         const unsigned g = (unsigned)(((long long)(d.nx + 1) * (d.ny + 1) * (d.nz + 1) + 255) / 256);
         bool par = false;
         for (int i = 0; i < 6; ++i) par = par || d.bf[i] >= 2;
-        if (par) k_edge<1><<<g, 256, 0, h->stream>>>(d);
-        else k_edge<0><<<g, 256, 0, h->stream>>>(d);
+        if (par) launch(k_edge<1>, g, 256, 0, h->stream, d.pdl, d);
+        else launch(k_edge<0>, g, 256, 0, h->stream, d.pdl, d);
     }
     h->launches++;
     if (h->cfg.fixpole && d.coord == 2) {
-        k_fixpole<<<(d.nx + 31) / 32, 256, 0, h->stream>>>(d);
+        launch(k_fixpole, (d.nx + 31) / 32, 256, 0, h->stream, d.pdl, d);
         h->launches++;
     }
     prof_end(h, PC_EMF);
@@ -1514,7 +1537,7 @@ static void enqueue_stage_b(cumc_handle *h, int stage, bool with_dt) {
         const long long cells = (long long)(d.nx + 1) * (d.ny + 1) * (d.nz + 1);
         const bool fp32 = h->cfg.precision == CUMC_FP32;
         if (fp32 && d.coord == 0 && d.source_kind == 0 && cells < (1LL << 31)) {
-            k_rk_cart<float><<<(unsigned)((cells + 255) / 256), 256, 0, h->stream>>>(d, stage);
+            launch(k_rk_cart<float>, (unsigned)((cells + 255) / 256), 256, 0, h->stream, d.pdl, d, stage);
         } else if (fp32) {
             launch_rk<float>(d, stage, cells, h->stream);
         } else {
@@ -1524,16 +1547,16 @@ static void enqueue_stage_b(cumc_handle *h, int stage, bool with_dt) {
     h->launches++;
     prof_end(h, PC_RK);
     prof_begin(h);
-    if (with_dt) k_recover<0, 1><<<cell_blocks(d), 256, 0, h->stream>>>(d, stage);
-    else k_recover<0, 0><<<cell_blocks(d), 256, 0, h->stream>>>(d, stage);
+    if (with_dt) launch(k_recover<0, 1>, cell_blocks(d), 256, 0, h->stream, d.pdl, d, stage);
+    else launch(k_recover<0, 0>, cell_blocks(d), 256, 0, h->stream, d.pdl, d, stage);
     h->launches++;
     prof_end(h, PC_RECOVER);
     prof_begin(h);
     launch_ghosts(h);
     prof_end(h, PC_BND);
     if (d.source_kind == 4) {
-        if (h->cfg.precision == CUMC_FP32) k_bh_update<float><<<1, 1024, 0, h->stream>>>(d, stage);
-        else k_bh_update<double><<<1, 1024, 0, h->stream>>>(d, stage);
+        if (h->cfg.precision == CUMC_FP32) launch(k_bh_update<float>, 1, 1024, 0, h->stream, d.pdl, d, stage);
+        else launch(k_bh_update<double>, 1, 1024, 0, h->stream, d.pdl, d, stage);
         h->launches++;
     }
 }
@@ -1541,8 +1564,8 @@ static void enqueue_stage_b(cumc_handle *h, int stage, bool with_dt) {
 static void enqueue_finddt(cumc_handle *h, int clamp) {
     const Dev &d = h->d;
     prof_begin(h);
-    k_finddt<<<cell_blocks(d), 256, 0, h->stream>>>(d);
-    k_dt_final<<<1, 1, 0, h->stream>>>(d, clamp);
+    launch(k_finddt, cell_blocks(d), 256, 0, h->stream, d.pdl, d);
+    launch(k_dt_final, 1, 1, 0, h->stream, d.pdl, d, clamp);
     h->launches += 2;
     prof_end(h, PC_DT);
 }
@@ -1552,7 +1575,7 @@ static void enqueue_finddt(cumc_handle *h, int clamp) {
 static void enqueue_step(cumc_handle *h, bool turn) {
     for (int s = 1; s <= 3; ++s) enqueue_stage(h, s, turn && s == 3);
     if (turn) {
-        k_step_turn<<<1, 1, 0, h->stream>>>(h->d);
+        launch(k_step_turn, 1, 1, 0, h->stream, h->d.pdl, h->d);
         h->launches++;
     }
 }
@@ -1640,7 +1663,10 @@ int cumc_create(const cumc_config *cfg, cumc_handle **out) {
     d.pos_fallback = cfg->positivity_fallback ? 1 : 0;
     d.tpb_recon = 256;
     d.tpb_riemann = 128;
-    d.riemann_minb = 1;
+    d.riemann_minb = 4;
+    // programmatic launches: 64^3 PPM 486 -> 467 us a step, 101 x 96 x 90 1379 ->
+    // 1354; below they cost (24^3 128 -> 161, 64^2 104 -> 124)
+    d.pdl = N3 >= 200000 ? 1 : 0;
     d.gamma = cfg->model.gamma; d.cfl = cfg->cfl;
     d.floor_kind = cfg->model.floor_kind; d.source_kind = cfg->model.source_kind; d.bc_kind = cfg->model.bc_kind;
     d.rho_floor = cfg->model.rho_floor; d.eps_floor = cfg->model.eps_floor; d.p_floor = cfg->model.p_floor;
@@ -1807,6 +1833,15 @@ int cumc_create(const cumc_config *cfg, cumc_handle **out) {
     cudaMemcpy(d.S, &s0, sizeof s0, cudaMemcpyHostToDevice);
     // flux kernels need more than 48 KB of dynamic shared memory only for large tiles
     default_flux_blocks(h);
+    // launch shapes of a handle that is not autotuned (measured over tubes of 100
+    // to 4000 zones, 64^2 to 600^2 and 24^3 to 101 x 96 x 90, PPM and WENO, both
+    // precisions): up to 32768 cells a sweep cannot fill the GPU and the fused
+    // kernel saves a launch (24^3 PPM FP64 128 against 146 us a step; 40^3, 247
+    // against 196 the other way); above, staged tiles (101 x 96 x 90 PPM FP64 1366
+    // against 1643 us with per-cell loads) unless a row fills its 32-cell tiles
+    // badly (40^3 WENO 268 against 222)
+    h->flux_mode = cfg->precision == CUMC_FP64 && (long long)nx * ny * nz <= 32768 ? 0 : 1;
+    d.recon_tile = 4 * nx >= 3 * 32 * ((nx + 31) / 32) ? 4 : 0;
     if (cudaDeviceSynchronize() != cudaSuccess) {
         g_create_err = "device setup failed";
         cumc_destroy(h);
@@ -1819,8 +1854,7 @@ int cumc_create(const cumc_config *cfg, cumc_handle **out) {
 int cumc_destroy(cumc_handle *h) {
     if (!h) return CUMC_OK;
     if (h->stream) cudaStreamSynchronize(h->stream);
-    if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
-    if (h->graph) cudaGraphDestroy(h->graph);
+    drop_graphs(h);
     if (h->sor_exec) cudaGraphExecDestroy(h->sor_exec);
     if (h->sor_graph) cudaGraphDestroy(h->sor_graph);
     if (h->snap_stream) {  // a snapshot copy in flight reads the staging buffer
@@ -1906,7 +1940,7 @@ int cumc_get_array(cumc_handle *h, int which, double *out, size_t n_doubles) {
 // INITIAL_UPDATE (initial.f90:86-116): CHECKRHO, FROMRVETOU, BOUNDARY, UPDATE
 static void enqueue_initial(cumc_handle *h) {
     const Dev &d = h->d;
-    k_recover<1, 0><<<cell_blocks(d), 256, 0, h->stream>>>(d, 0);
+    launch(k_recover<1, 0>, cell_blocks(d), 256, 0, h->stream, d.pdl, d, 0);
     h->launches++;
     launch_ghosts(h);
 }
@@ -1935,6 +1969,19 @@ int cumc_finddt(cumc_handle *h, double *dt) {
     return CUMC_OK;
 }
 
+// capture one step (which: cumc_handle::graph) the first time
+static int step_graph(cumc_handle *h, int which) {
+    if (h->graph_exec[which]) return CUMC_OK;
+    const int64_t before = h->launches;
+    CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+    enqueue_step(h, which == 0);
+    CK(cudaStreamEndCapture(h->stream, &h->graph[which]));
+    CK(cudaGraphInstantiate(&h->graph_exec[which], h->graph[which], 0));
+    h->kernels_per_step[which] = (int)(h->launches - before);
+    h->launches = before;
+    return CUMC_OK;
+}
+
 int cumc_rk3_step(cumc_handle *h, double dt) {
     Range r("cumc RUNGEKUTTA");
     if (!h) return fail(h, CUMC_EINVAL, "null handle");
@@ -1943,7 +1990,17 @@ int cumc_rk3_step(cumc_handle *h, double dt) {
     if (h->d.source_kind == CUMC_SRC_COLLAPSAR && !h->d.phi[0])
         return fail(h, CUMC_ENOTREADY, "the collapsar source needs cumc_poisson_setup first");
     CK(cudaMemcpyAsync(&h->d.S->dt, &dt, sizeof(double), cudaMemcpyHostToDevice, h->stream));
-    enqueue_step(h, false);
+    // a program that steps by itself pays for a captured step once it has taken
+    // two: 24 to 33 launches from the host cost more than such a step runs on a
+    // small grid
+    if (h->eager_steps < 2) {
+        ++h->eager_steps;
+        enqueue_step(h, false);
+    } else {
+        if (int rc = step_graph(h, 1)) return rc;
+        CK(cudaGraphLaunch(h->graph_exec[1], h->stream));
+        h->launches += h->kernels_per_step[1];
+    }
     CK(cudaGetLastError());
     return check_scalars(h);
 }
@@ -1969,24 +2026,15 @@ int cumc_evolve(cumc_handle *h, double t_end, int max_steps, double *t_inout, in
     s.dt_bits = (unsigned long long)0x40F86A0000000000ull;  // bits of 1.0e5
     *h->S_host = s;
     CK(cudaMemcpyAsync(h->d.S, h->S_host, sizeof(Scalars), cudaMemcpyHostToDevice, h->stream));
-    // capture one step the first time
-    if (!h->graph_exec) {
-        int64_t before = h->launches;
-        CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        enqueue_step(h, true);
-        CK(cudaStreamEndCapture(h->stream, &h->graph));
-        CK(cudaGraphInstantiate(&h->graph_exec, h->graph, 0));
-        h->kernels_per_step = (int)(h->launches - before);
-        h->launches = before;
-    }
+    if (int rc = step_graph(h, 0)) return rc;
     enqueue_finddt(h, 1);  // the first step's dt; each step's turn makes the next
     // replay in chunks; kernels turn into no-ops once the device sets done
     int issued = 0;
     while (true) {
         int chunk = max_steps - issued;
         if (chunk > 64) chunk = 64;
-        for (int i = 0; i < chunk; ++i) CK(cudaGraphLaunch(h->graph_exec, h->stream));
-        h->launches += (int64_t)chunk * h->kernels_per_step;
+        for (int i = 0; i < chunk; ++i) CK(cudaGraphLaunch(h->graph_exec[0], h->stream));
+        h->launches += (int64_t)chunk * h->kernels_per_step[0];
         issued += chunk;
         CK(cudaMemcpyAsync(h->S_host, h->d.S, sizeof(Scalars), cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));
@@ -2108,8 +2156,7 @@ int cumc_autotune(cumc_handle *h, int *choice_out, double *best_ms_out) {
     h->d.riemann_minb = all[bi].minb;
     h->d.recon_tile = all[bi].tile;
     // a captured step holds the old launch shapes
-    if (h->graph_exec) { cudaGraphExecDestroy(h->graph_exec); h->graph_exec = nullptr; }
-    if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
+    drop_graphs(h);
     if (choice_out) {
         choice_out[0] = all[bi].mode; choice_out[1] = all[bi].tpb_recon;
         choice_out[2] = all[bi].tpb_riemann; choice_out[3] = all[bi].minb;
@@ -2133,8 +2180,7 @@ int cumc_set_tuning(cumc_handle *h, const int *choice) {
     h->d.tpb_recon = choice[1];
     h->d.tpb_riemann = choice[2];
     h->d.riemann_minb = choice[3];
-    if (h->graph_exec) { cudaGraphExecDestroy(h->graph_exec); h->graph_exec = nullptr; }
-    if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
+    drop_graphs(h);
     return CUMC_OK;
 }
 
@@ -2152,8 +2198,7 @@ int cumc_fallback_count(cumc_handle *h, int enable, unsigned long long *count_ou
     if (want != h->d.fb_count) {
         h->d.fb_count = want;
         // the captured step holds the kernels' parameters: capture it again
-        if (h->graph_exec) { cudaGraphExecDestroy(h->graph_exec); h->graph_exec = nullptr; }
-        if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
+        drop_graphs(h);
     }
     if (count_out) {
         *count_out = 0;
@@ -2180,9 +2225,9 @@ int cumc_set_concurrent_sweeps(cumc_handle *h, int on) {
         for (int i = 0; i < 3; ++i) CK(cudaEventCreateWithFlags(&h->fev[i], cudaEventDisableTiming));
     }
     h->sweeps_concurrent = on != 0;
+    h->d.pdl = !on && h->d.N3 >= 200000 ? 1 : 0;  // a kernel after a join has several predecessors
     // a captured step graph holds the old launch order
-    if (h->graph_exec) { cudaGraphExecDestroy(h->graph_exec); h->graph_exec = nullptr; }
-    if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
+    drop_graphs(h);
     return CUMC_OK;
 }
 
@@ -2214,8 +2259,7 @@ int cumc_learn_set(cumc_handle *h, const float *params, float threshold, int fla
     d.audit_interval = audit_interval;
     d.audit_tol = audit_tol;
     // the captured step holds the kernel arguments: capture again
-    if (h->graph_exec) { cudaGraphExecDestroy(h->graph_exec); h->graph_exec = nullptr; }
-    if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
+    drop_graphs(h);
     return CUMC_OK;
 }
 
@@ -2305,8 +2349,7 @@ int cumc_poisson_setup(cumc_handle *h, double rho_atm, double omega) {
     h->d.phi[0] = s.phi[0];
     h->d.phi[1] = s.phi[1];
     h->d.phx = s.hx;
-    if (h->graph_exec) { cudaGraphExecDestroy(h->graph_exec); h->graph_exec = nullptr; }
-    if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
+    drop_graphs(h);
     // the initial model's guess: phi = 0 everywhere, ghosts included (custom.f90:498-507)
     for (int c = 0; c < 2; ++c) CK(cudaMemsetAsync(s.phi[c], 0, half * sizeof(double), h->stream));
     // omega lives in the captured kernel parameters: capture again
@@ -2747,8 +2790,7 @@ int cumc_collapsar_set(cumc_handle *h, double m_bh, double c_code) {
     CK(cudaStreamSynchronize(h->stream));
     if (h->d.c_code != c_code) {
         h->d.c_code = c_code;
-        if (h->graph_exec) { cudaGraphExecDestroy(h->graph_exec); h->graph_exec = nullptr; }
-        if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
+        drop_graphs(h);
     }
     return CUMC_OK;
 }

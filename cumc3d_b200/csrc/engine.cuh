@@ -49,6 +49,7 @@ struct Dev {
     int tpb_recon, tpb_riemann;  // threads per block of the split flux kernels (autotuned)
     int riemann_minb;            // blocks/SM the Riemann kernel is compiled for (1, 4, 5, 6; 14, 15, 16:
                                  // the prefetching kernel at 4, 5, 6; autotuned)
+    int pdl;                     // launch() with programmatic dependence (not with concurrent sweeps)
     int recon_tile;              // 0: per-cell stencil loads; 1, 2: staged tiles, cells per thread (autotuned)
     int wuni[3];                 // 1: the axis's reconstruction weights are identical in every cell
     double wu[3][14];            // those weights (FP64 form)
@@ -106,6 +107,28 @@ struct Dev {
     // sweeps and stages (null: not counted; cumc_fallback_count)
     unsigned long long *fb_count;
 };
+
+// The stage kernels are launched programmatically dependent: a kernel's CTAs may
+// be placed while the one before drains, and wait here until its writes are
+// visible (every stage kernel begins with this, so the order is transitive).
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+static inline void launch(void (*k)(P...), dim3 g, dim3 b, size_t smem, cudaStream_t s, int pdl, const A &...a) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = g;
+    c.blockDim = b;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    c.numAttrs = pdl ? 1 : 0;
+    cudaLaunchKernelEx(&c, k, P(a)...);
+}
 
 __device__ __forceinline__ int cidx(const Dev &d, int j, int k, int l) {
     return (j + 2) + d.NX * ((k + 2) + d.NY * (l + 2));

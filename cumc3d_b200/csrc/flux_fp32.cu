@@ -33,12 +33,12 @@ static void launch_learned_dir(const Dev &d, int rs, int stage, cudaStream_t s) 
     const dim3 tb(32, 8, 1);
     if (d.recon_tile == 1) {
         const dim3 g = recon_tile_grid(d, DIR, 1);
-        if (d.wuni[DIR]) k_recon_tile<float, DIR, REC_WENO, 1, 1, 1><<<g, tb, 0, s>>>(d, stage);
-        else k_recon_tile<float, DIR, REC_WENO, 0, 1, 1><<<g, tb, 0, s>>>(d, stage);
+        if (d.wuni[DIR]) launch(k_recon_tile<float, DIR, REC_WENO, 1, 1, 1>, g, tb, 0, s, d.pdl, d, stage);
+        else launch(k_recon_tile<float, DIR, REC_WENO, 0, 1, 1>, g, tb, 0, s, d.pdl, d, stage);
     } else {
         const dim3 g = recon_tile_grid(d, DIR, 2);
-        if (d.wuni[DIR]) k_recon_tile<float, DIR, REC_WENO, 1, 2, 1><<<g, tb, 0, s>>>(d, stage);
-        else k_recon_tile<float, DIR, REC_WENO, 0, 2, 1><<<g, tb, 0, s>>>(d, stage);
+        if (d.wuni[DIR]) launch(k_recon_tile<float, DIR, REC_WENO, 1, 2, 1>, g, tb, 0, s, d.pdl, d, stage);
+        else launch(k_recon_tile<float, DIR, REC_WENO, 0, 2, 1>, g, tb, 0, s, d.pdl, d, stage);
     }
     dim3 g, b;
     split_dims(d, DIR, false, g, b);

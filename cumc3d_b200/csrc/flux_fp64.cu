@@ -11,6 +11,7 @@ void launch_flux_fp64(const Dev &d, int dir, int rec, int rs, dim3 grid, dim3 bl
 // the faces the sweeps of a stage left on the list, with the plain HLLD; the
 // list is emptied by the next kernel of the stage (k_edge)
 __global__ void __launch_bounds__(128) k_faces_deferred(const Dev d) {
+    pdl_wait();
     if (d.S->done) return;
     const unsigned n = *d.fix_n < d.fix_cap ? *d.fix_n : d.fix_cap;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -33,7 +34,7 @@ __global__ void __launch_bounds__(128) k_faces_deferred(const Dev d) {
 }
 void launch_faces_deferred(const Dev &d, cudaStream_t s) {
     const unsigned most = 4u * (unsigned)d.num_sms, want = (d.fix_cap + 127u) / 128u;
-    k_faces_deferred<<<want < most ? want : most, 128, 0, s>>>(d);
+    launch(k_faces_deferred, want < most ? want : most, 128, 0, s, d.pdl, d);
 }
 void launch_split_fp64(const Dev &d, int dir, int rec, int rs, cudaStream_t s, const TmaMaps *tma) {
     launch_split_t<double>(d, dir, rec, rs, s, tma);
@@ -47,12 +48,12 @@ static void launch_learned64_dir(const Dev &d, int rs, int stage, cudaStream_t s
     const dim3 tb(32, 8, 1);
     if (d.recon_tile == 2) {
         const dim3 g = recon_tile_grid(d, DIR, 2);
-        if (d.wuni[DIR]) k_recon_tile<double, DIR, REC_WENO, 1, 2, 2, 2><<<g, tb, 0, s>>>(d, stage);
-        else k_recon_tile<double, DIR, REC_WENO, 0, 2, 2, 2><<<g, tb, 0, s>>>(d, stage);
+        if (d.wuni[DIR]) launch(k_recon_tile<double, DIR, REC_WENO, 1, 2, 2, 2>, g, tb, 0, s, d.pdl, d, stage);
+        else launch(k_recon_tile<double, DIR, REC_WENO, 0, 2, 2, 2>, g, tb, 0, s, d.pdl, d, stage);
     } else {
         const dim3 g = recon_tile_grid(d, DIR, 1);
-        if (d.wuni[DIR]) k_recon_tile<double, DIR, REC_WENO, 1, 1, 2, 3><<<g, tb, 0, s>>>(d, stage);
-        else k_recon_tile<double, DIR, REC_WENO, 0, 1, 2, 3><<<g, tb, 0, s>>>(d, stage);
+        if (d.wuni[DIR]) launch(k_recon_tile<double, DIR, REC_WENO, 1, 1, 2, 3>, g, tb, 0, s, d.pdl, d, stage);
+        else launch(k_recon_tile<double, DIR, REC_WENO, 0, 1, 2, 3>, g, tb, 0, s, d.pdl, d, stage);
     }
     dim3 g, b;
     split_dims(d, DIR, false, g, b);

@@ -197,6 +197,7 @@ template <> __device__ __forceinline__ const float *weights<float>(const Dev &d,
 
 template <class T, int DIR, int REC, int RS>
 __global__ void __launch_bounds__(256) k_flux(const Dev d) {
+    pdl_wait();
     if (d.S->done) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int nthr = blockDim.x * blockDim.y;
@@ -314,6 +315,7 @@ template <> __device__ __forceinline__ float uni_w<float>(const Dev &d, int dir,
 // kernel parameters and live in uniform registers.
 template <class T, int DIR, int REC, int UNI>
 __global__ void __launch_bounds__(256, sizeof(T) == 8 && REC == REC_WENO ? 2 : 1) k_recon(const Dev d) {
+    pdl_wait();
     if (d.S->done) return;
     // one thread per reconstructed cell, enumerated x fastest with no tail
     // padding per row: x extent nx+2 (x sweep) or nx, then y, then z
@@ -359,6 +361,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 && REC == REC_WENO ? 2 : 1
 
 template <class T, int DIR, int RS, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_riemann(const Dev d) {
+    pdl_wait();
     if (d.S->done) return;
     int f, j, k, l, ns;
     {
@@ -410,6 +413,7 @@ __device__ __forceinline__ void cp_async_elem(void *smem, const void *gmem, int 
 
 template <class T, int DIR, int RS, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_riemann_pf(const Dev d) {
+    pdl_wait();
     if (d.S->done) return;
     __shared__ T qb[2][14][128];
     __shared__ double bb[2][128];
@@ -495,11 +499,11 @@ static void launch_recon_tile_c(const Dev &d, int rec, cudaStream_t s) {
     constexpr bool W = sizeof(T) == sizeof(double);
     constexpr int M = KIND == 4 ? 4 : 1, MW = !W ? M : KIND == 4 ? 3 : 2;
     switch (rec) {
-        case REC_TVD_MM: k_recon_tile<T, DIR, REC_TVD_MM, UNI, CPT, 0, M><<<g, b, 0, s>>>(d); break;
-        case REC_TVD_VL: k_recon_tile<T, DIR, REC_TVD_VL, UNI, CPT, 0, M><<<g, b, 0, s>>>(d); break;
-        case REC_TVD_MC: k_recon_tile<T, DIR, REC_TVD_MC, UNI, CPT, 0, M><<<g, b, 0, s>>>(d); break;
-        case REC_PPM: k_recon_tile<T, DIR, REC_PPM, UNI, CPT, 0, M><<<g, b, 0, s>>>(d); break;
-        default: k_recon_tile<T, DIR, REC_WENO, UNI, CPT, 0, MW><<<g, b, 0, s>>>(d); break;
+        case REC_TVD_MM: launch(k_recon_tile<T, DIR, REC_TVD_MM, UNI, CPT, 0, M>, g, b, 0, s, d.pdl, d, 0); break;
+        case REC_TVD_VL: launch(k_recon_tile<T, DIR, REC_TVD_VL, UNI, CPT, 0, M>, g, b, 0, s, d.pdl, d, 0); break;
+        case REC_TVD_MC: launch(k_recon_tile<T, DIR, REC_TVD_MC, UNI, CPT, 0, M>, g, b, 0, s, d.pdl, d, 0); break;
+        case REC_PPM: launch(k_recon_tile<T, DIR, REC_PPM, UNI, CPT, 0, M>, g, b, 0, s, d.pdl, d, 0); break;
+        default: launch(k_recon_tile<T, DIR, REC_WENO, UNI, CPT, 0, MW>, g, b, 0, s, d.pdl, d, 0); break;
     }
 }
 // recon_tile: 1, 2 staged tiles with 1 or 2 cells per thread; 4 one cell per
@@ -519,11 +523,11 @@ static void launch_recon_u(const Dev &d, int rec, dim3 g, dim3 b, cudaStream_t s
         return;
     }
     switch (rec) {
-        case REC_TVD_MM: k_recon<T, DIR, REC_TVD_MM, UNI><<<g, b, 0, s>>>(d); break;
-        case REC_TVD_VL: k_recon<T, DIR, REC_TVD_VL, UNI><<<g, b, 0, s>>>(d); break;
-        case REC_TVD_MC: k_recon<T, DIR, REC_TVD_MC, UNI><<<g, b, 0, s>>>(d); break;
-        case REC_PPM: k_recon<T, DIR, REC_PPM, UNI><<<g, b, 0, s>>>(d); break;
-        default: k_recon<T, DIR, REC_WENO, UNI><<<g, b, 0, s>>>(d); break;
+        case REC_TVD_MM: launch(k_recon<T, DIR, REC_TVD_MM, UNI>, g, b, 0, s, d.pdl, d); break;
+        case REC_TVD_VL: launch(k_recon<T, DIR, REC_TVD_VL, UNI>, g, b, 0, s, d.pdl, d); break;
+        case REC_TVD_MC: launch(k_recon<T, DIR, REC_TVD_MC, UNI>, g, b, 0, s, d.pdl, d); break;
+        case REC_PPM: launch(k_recon<T, DIR, REC_PPM, UNI>, g, b, 0, s, d.pdl, d); break;
+        default: launch(k_recon<T, DIR, REC_WENO, UNI>, g, b, 0, s, d.pdl, d); break;
     }
 }
 // riemann_minb 14, 15, 16: the prefetching kernel at 4, 5, 6 blocks per SM
@@ -536,19 +540,19 @@ static void launch_riemann_pf(const Dev &d, int rs, cudaStream_t s) {
     if (nblk > need) nblk = need;
     const dim3 g((unsigned)nblk), b(128);
     switch (rs) {
-        case RS_LF: k_riemann_pf<T, DIR, RS_LF, MINB><<<g, b, 0, s>>>(d); break;
-        case RS_HLL: k_riemann_pf<T, DIR, RS_HLL, MINB><<<g, b, 0, s>>>(d); break;
-        case RS_HLLC: k_riemann_pf<T, DIR, RS_HLLC, MINB><<<g, b, 0, s>>>(d); break;
-        default: k_riemann_pf<T, DIR, RS_HLLD, MINB><<<g, b, 0, s>>>(d); break;
+        case RS_LF: launch(k_riemann_pf<T, DIR, RS_LF, MINB>, g, b, 0, s, d.pdl, d); break;
+        case RS_HLL: launch(k_riemann_pf<T, DIR, RS_HLL, MINB>, g, b, 0, s, d.pdl, d); break;
+        case RS_HLLC: launch(k_riemann_pf<T, DIR, RS_HLLC, MINB>, g, b, 0, s, d.pdl, d); break;
+        default: launch(k_riemann_pf<T, DIR, RS_HLLD, MINB>, g, b, 0, s, d.pdl, d); break;
     }
 }
 template <class T, int DIR, int MINB>
 static void launch_riemann_m(const Dev &d, int rs, dim3 g, dim3 b, cudaStream_t s) {
     switch (rs) {
-        case RS_LF: k_riemann<T, DIR, RS_LF, MINB><<<g, b, 0, s>>>(d); break;
-        case RS_HLL: k_riemann<T, DIR, RS_HLL, MINB><<<g, b, 0, s>>>(d); break;
-        case RS_HLLC: k_riemann<T, DIR, RS_HLLC, MINB><<<g, b, 0, s>>>(d); break;
-        default: k_riemann<T, DIR, RS_HLLD, MINB><<<g, b, 0, s>>>(d); break;
+        case RS_LF: launch(k_riemann<T, DIR, RS_LF, MINB>, g, b, 0, s, d.pdl, d); break;
+        case RS_HLL: launch(k_riemann<T, DIR, RS_HLL, MINB>, g, b, 0, s, d.pdl, d); break;
+        case RS_HLLC: launch(k_riemann<T, DIR, RS_HLLC, MINB>, g, b, 0, s, d.pdl, d); break;
+        default: launch(k_riemann<T, DIR, RS_HLLD, MINB>, g, b, 0, s, d.pdl, d); break;
     }
 }
 // the TMA-staged reconstruction: persistent CTAs, as many as fit on the GPU
@@ -566,7 +570,7 @@ static void launch_recon_tma_r(const Dev &d, const TmaMaps &tm, cudaStream_t s) 
     const long long ntiles = (long long)tg.x * tg.y * tg.z;
     long long nblk = (long long)d.num_sms * per_sm;
     if (nblk > ntiles) nblk = ntiles;
-    k_recon_tma<DIR, REC, UNI><<<(unsigned)nblk, dim3(32, 8, 1), TmaBox<DIR>::SMEM, s>>>(d, tm);
+    launch(k_recon_tma<DIR, REC, UNI>, (unsigned)nblk, dim3(32, 8, 1), TmaBox<DIR>::SMEM, s, d.pdl, d, tm);
 }
 template <int DIR, int UNI>
 static void launch_recon_tma(const Dev &d, int rec, const TmaMaps &tm, cudaStream_t s) {
@@ -624,10 +628,10 @@ static void launch_rs(const Dev &d, int rs, dim3 g, dim3 b, size_t sm, cudaStrea
         default: flux_smem<T, DIR, REC, RS_HLLD>(sm); break;
     }
     switch (rs) {
-        case RS_LF: k_flux<T, DIR, REC, RS_LF><<<g, b, sm, s>>>(d); break;
-        case RS_HLL: k_flux<T, DIR, REC, RS_HLL><<<g, b, sm, s>>>(d); break;
-        case RS_HLLC: k_flux<T, DIR, REC, RS_HLLC><<<g, b, sm, s>>>(d); break;
-        default: k_flux<T, DIR, REC, RS_HLLD><<<g, b, sm, s>>>(d); break;
+        case RS_LF: launch(k_flux<T, DIR, REC, RS_LF>, g, b, sm, s, d.pdl, d); break;
+        case RS_HLL: launch(k_flux<T, DIR, REC, RS_HLL>, g, b, sm, s, d.pdl, d); break;
+        case RS_HLLC: launch(k_flux<T, DIR, REC, RS_HLLC>, g, b, sm, s, d.pdl, d); break;
+        default: launch(k_flux<T, DIR, REC, RS_HLLD>, g, b, sm, s, d.pdl, d); break;
     }
 }
 template <class T, int DIR>

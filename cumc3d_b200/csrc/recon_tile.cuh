@@ -162,6 +162,7 @@ __device__ __forceinline__ void recon_tile_cells(const Dev &d, const T *__restri
 // resident warps)
 template <class T, int DIR, int REC, int UNI, int CPT, int LRN = 0, int MINB = 1>
 __global__ void __launch_bounds__(256, MINB) k_recon_tile(const Dev d, int stage = 0) {
+    pdl_wait();
     if (d.S->done) return;
     if (LRN == 1 && learned_refresh_stage(d, stage)) return;  // the network kernel reconstructs this stage
     constexpr int TX = 32, TY = 8;
@@ -263,6 +264,7 @@ __device__ __forceinline__ void tma_issue(const TmaMaps &maps, double *buf, unsi
 
 template <int DIR, int REC, int UNI>
 __global__ void __launch_bounds__(256) k_recon_tma(const Dev d, const __grid_constant__ TmaMaps maps) {
+    pdl_wait();
     if (d.S->done) return;
     using B = TmaBox<DIR>;
     extern __shared__ __align__(16) unsigned char tma_raw[];
