@@ -27,6 +27,9 @@ struct cumc_batch {
     int cluster_size = BATCH_CLUSTER;  // CTAs that share one large problem
     int coop_min_n = -1;               // set by cumc_batch_set_cluster; -1: chosen per run
     int64_t launches = 0;
+    std::vector<int> sorted_n;         // problem sizes in launch order, largest first
+    cudaStream_t aux[4] = {};          // one size class each, beside `stream`
+    cudaEvent_t fork = nullptr, join[4] = {};
 };
 
 static std::string g_batch_err;
@@ -80,6 +83,7 @@ int cumc_batch_create(const cumc_batch_config *cfg, cumc_batch **out) {
     std::vector<int> order(b->nprob);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return b->n[a] > b->n[c]; });
+    for (int p : order) b->sorted_n.push_back(b->n[p]);
     std::vector<BatchProblem> prob(b->nprob);
     for (int p = 0; p < b->nprob; ++p) {
         memset(&prob[p], 0, sizeof(BatchProblem));
@@ -138,6 +142,11 @@ int cumc_batch_destroy(cumc_batch *b) {
     if (!b) return CUMC_OK;
     if (b->stream) cudaStreamSynchronize(b->stream);
     for (void *p : b->allocs) cudaFree(p);
+    for (int i = 0; i < 4; ++i) {
+        if (b->aux[i]) cudaStreamDestroy(b->aux[i]);
+        if (b->join[i]) cudaEventDestroy(b->join[i]);
+    }
+    if (b->fork) cudaEventDestroy(b->fork);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
     return CUMC_OK;
@@ -184,30 +193,106 @@ int cumc_batch_get_state(cumc_batch *b, int p, double *prim_row, double *eps_row
     return CUMC_OK;
 }
 
-int cumc_batch_run(cumc_batch *b, int max_steps, double *t_out, int *steps_out, int *status_out) {
-    if (!b) return bfail(b, CUMC_EINVAL, "null batch");
-    b->d.max_steps = max_steps > 0 ? max_steps : 0x7fffffff;
-    if (cudaMemsetAsync(b->d.next, 0, sizeof(int), b->stream) != cudaSuccess) return bfail(b, CUMC_ECUDA, "memset failed");
+// the first `count` problems (the largest) through the persistent kernel, whose
+// rows live in global memory: any size, any sharing
+static cudaError_t run_persistent(cumc_batch *b, int count) {
+    if (cudaMemsetAsync(b->d.next, 0, sizeof(int), b->stream) != cudaSuccess) return cudaErrorUnknown;
+    BatchDev d = b->d;
+    d.nprob = count;
     // sharing threshold: a batch no larger than the clusters that can be
     // resident at once (two 256-thread CTAs per SM) leaves SMs idle, so its
     // problems are shared from 256 cells up (one cell per thread and fewer
     // steps' worth of latency); a larger one shares only its largest problems
     if (b->coop_min_n < 0) {
         const int resident = b->cluster_size > 1 ? 2 * b->sm_count / b->cluster_size : 2 * b->sm_count;
-        b->d.coop_min_n = b->nprob <= resident ? BATCH_COOP_MIN_N_FEW : BATCH_COOP_MIN_N;
+        d.coop_min_n = count <= resident ? BATCH_COOP_MIN_N_FEW : BATCH_COOP_MIN_N;
     } else {
-        b->d.coop_min_n = b->coop_min_n;
+        d.coop_min_n = b->coop_min_n;
     }
-    cudaError_t e = b->precision == CUMC_FP32
-                        ? launch_batch_fp32(b->d, b->recon, b->riemann, 0, b->cluster_size, b->stream)
-                        : launch_batch_fp64(b->d, b->recon, b->riemann, 0, b->cluster_size, b->stream);
+    auto go = [&](int cluster) {
+        return b->precision == CUMC_FP32 ? launch_batch_fp32(d, b->recon, b->riemann, 0, cluster, b->stream)
+                                         : launch_batch_fp64(d, b->recon, b->riemann, 0, cluster, b->stream);
+    };
+    cudaError_t e = go(b->cluster_size);
     if (e == cudaErrorInvalidConfiguration || e == cudaErrorInvalidValue) {
         cudaGetLastError();  // no room for a cluster: one CTA per problem
-        e = b->precision == CUMC_FP32 ? launch_batch_fp32(b->d, b->recon, b->riemann, 0, 1, b->stream)
-                                      : launch_batch_fp64(b->d, b->recon, b->riemann, 0, 1, b->stream);
+        e = go(1);
     }
+    if (e == cudaSuccess) b->launches++;
+    return e;
+}
+
+// Every problem of up to 16 x 254 cells on a cluster of its own, one cell per
+// thread (tube_kernel.cuh): the fewest CTAs that hold it, a power of two, and
+// while the whole batch leaves half the SMs idle twice as many (up to 8, at
+// least 16 cells each), since a CTA with fewer warps runs a stage sooner.
+// Problems with the same cluster are neighbours in the launch order; each such
+// class is one launch on a stream of its own, the largest first.  What does not
+// fit goes to the persistent kernel.
+static cudaError_t run_tubes(cumc_batch *b) {
+    const int np = b->nprob;
+    auto ctas = [&](int n) {
+        int c = 1;
+        while (c < 16 && (n + c - 1) / c > TUBE_MOST_CELLS) c *= 2;
+        return c;
+    };
+    int big = 0;  // problems beyond 16 CTAs
+    while (big < np && b->sorted_n[big] > 16 * TUBE_MOST_CELLS) ++big;
+    long long total = 0;
+    for (int p = big; p < np; ++p) total += ctas(b->sorted_n[p]);
+    int wider = 1;
+    while (wider < 8 && 2 * wider * total <= b->sm_count) wider *= 2;
+    auto size_of = [&](int n) {
+        int c = ctas(n);
+        for (int w = wider; w > 1 && c < 8 && n / (2 * c) >= 16; w /= 2) c *= 2;
+        return c;
+    };
+    if (!b->fork) {
+        cudaError_t e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
+        for (int i = 0; i < 4 && e == cudaSuccess; ++i) {
+            e = cudaStreamCreateWithFlags(&b->aux[i], cudaStreamNonBlocking);
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join[i], cudaEventDisableTiming);
+        }
+        if (e != cudaSuccess) return e;
+    }
+    cudaError_t e = cudaEventRecord(b->fork, b->stream);
+    int used = 0;
+    for (int p = big; p < np && e == cudaSuccess;) {
+        const int size = size_of(b->sorted_n[p]);
+        int q = p;
+        while (q < np && size_of(b->sorted_n[q]) == size) ++q;
+        cudaStream_t st = used < 4 ? b->aux[used] : b->stream;
+        if (used < 4) e = cudaStreamWaitEvent(st, b->fork, 0);
+        if (e == cudaSuccess)
+            e = b->precision == CUMC_FP32 ? launch_tube_fp32(b->d, b->recon, b->riemann, p, q - p, size, st)
+                                          : launch_tube_fp64(b->d, b->recon, b->riemann, p, q - p, size, st);
+        if (e != cudaSuccess && size == 16 && p == big) {
+            cudaGetLastError();  // no room for a 16-CTA cluster
+            big = p = q;
+            e = cudaSuccess;
+            continue;
+        }
+        b->launches++;
+        if (used < 4 && e == cudaSuccess) {
+            e = cudaEventRecord(b->join[used], st);
+            ++used;
+        }
+        p = q;
+    }
+    if (e == cudaSuccess && big > 0) e = run_persistent(b, big);
+    for (int i = 0; i < used; ++i) {
+        const cudaError_t w = cudaStreamWaitEvent(b->stream, b->join[i], 0);
+        if (e == cudaSuccess) e = w;
+    }
+    return e;
+}
+
+int cumc_batch_run(cumc_batch *b, int max_steps, double *t_out, int *steps_out, int *status_out) {
+    if (!b) return bfail(b, CUMC_EINVAL, "null batch");
+    b->d.max_steps = max_steps > 0 ? max_steps : 0x7fffffff;
+    // cumc_batch_set_cluster's shape belongs to the persistent kernel
+    const cudaError_t e = b->coop_min_n < 0 ? run_tubes(b) : run_persistent(b, b->nprob);
     if (e != cudaSuccess) return bfail(b, CUMC_ECUDA, std::string("batch launch: ") + cudaGetErrorString(e));
-    b->launches++;
     if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(b->stream) != cudaSuccess)
         return bfail(b, CUMC_ECUDA, "batch kernel failed");
     std::vector<BatchProblem> prob(b->nprob);

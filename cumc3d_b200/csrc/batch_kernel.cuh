@@ -88,6 +88,18 @@ __device__ __forceinline__ double bmin_block(double v, double *red) {
     return r;
 }
 
+// x^2 + y^2 + z^2 and the conserved energy of the recovery.  FP64 form: the
+// reference's roundings.  The FP32 form is built with contraction; its roundings
+// are written out, so that both batch kernels (and every build) agree.
+template <class T>
+__device__ __forceinline__ double sum_sq(double x, double y, double z) {
+    if (sizeof(T) == sizeof(double)) return __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z));
+    return __fma_rn(z, z, __fma_rn(x, x, __dmul_rn(y, y)));
+}
+__device__ __forceinline__ double energy(double rho, double e, double vsquare, double bsquare) {
+    return __dadd_rn(__dmul_rn(rho, __dadd_rn(e, 0.5 * vsquare)), 0.5 * bsquare);
+}
+
 // floors of model/riemann/src/custom.f90:103-127 (eps >= 0)
 __device__ __forceinline__ void batch_floor(const BatchDev &b, double &e) {
     if (b.floor_kind == 1) e = dmax(e, 0.0);
@@ -144,13 +156,13 @@ __device__ __forceinline__ void batch_problem(const BatchDev &b, BatchShared &sh
         const double bx = 0.5 * (bxf + bxm);
         const double by = 0.5 * (by1 + by0);
         const double bz = 0.5 * (bz1 + bz0);
-        const double vsquare = vx * vx + vy * vy + vz * vz;
-        const double bsquare = bx * bx + by * by + bz * bz;
+        const double vsquare = sum_sq<T>(vx, vy, vz);
+        const double bsquare = sum_sq<T>(bx, by, bz);
         b.U[0][c] = rho;
         b.U[1][c] = vx * rho;
         b.U[2][c] = vy * rho;
         b.U[3][c] = vz * rho;
-        b.U[4][c] = rho * (e + 0.5 * vsquare) + 0.5 * bsquare;
+        b.U[4][c] = energy(rho, e, vsquare, bsquare);
         b.BC[0][c] = bx;
         b.BC[1][c] = by;
         b.BC[2][c] = bz;
@@ -391,8 +403,8 @@ __device__ __forceinline__ void batch_problem(const BatchDev &b, BatchShared &sh
                 const double byu = 0.5 * (uby1 + uby0);
                 const double bzu = 0.5 * (ubz1 + ubz0);
                 const double vx = dv(u1, u0), vy = dv(u2, u0), vz = dv(u3, u0);
-                const double bsquare = bxu * bxu + byu * byu + bzu * bzu;
-                const double vsquare = vx * vx + vy * vy + vz * vz;
+                const double bsquare = sum_sq<T>(bxu, byu, bzu);
+                const double vsquare = sum_sq<T>(vx, vy, vz);
                 double e = (u4 - 0.5 * bsquare) / u0 - 0.5 * vsquare;
                 batch_floor(b, e);
                 if (stage == 3) batch_floor(b, e);
@@ -528,6 +540,12 @@ static cudaError_t launch_batch_t(const BatchDev &b, int rec, int rs, int cluste
     }
 #undef CUMC_BATCH_RS
 }
+
+// tube_kernel.cuh: problems first .. first + count - 1 of b.order, one cluster of
+// `size` CTAs each
+constexpr int TUBE_MOST_CELLS = 254;  // of one CTA
+cudaError_t launch_tube_fp64(const BatchDev &b, int rec, int rs, int first, int count, int size, cudaStream_t s);
+cudaError_t launch_tube_fp32(const BatchDev &b, int rec, int rs, int first, int count, int size, cudaStream_t s);
 
 // clusters <= 0: as many clusters of cluster_size CTAs as fit on the device
 cudaError_t launch_batch_fp64(const BatchDev &b, int rec, int rs, int clusters, int cluster_size, cudaStream_t s);
