@@ -28,8 +28,8 @@ struct cumc_batch {
     int coop_min_n = -1;               // set by cumc_batch_set_cluster; -1: chosen per run
     int64_t launches = 0;
     std::vector<int> sorted_n;         // problem sizes in launch order, largest first
-    cudaStream_t aux[4] = {};          // one size class each, beside `stream`
-    cudaEvent_t fork = nullptr, join[4] = {};
+    cudaStream_t aux[6] = {};          // one size class each, beside `stream`
+    cudaEvent_t fork = nullptr, join[6] = {};
 };
 
 static std::string g_batch_err;
@@ -142,7 +142,7 @@ int cumc_batch_destroy(cumc_batch *b) {
     if (!b) return CUMC_OK;
     if (b->stream) cudaStreamSynchronize(b->stream);
     for (void *p : b->allocs) cudaFree(p);
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < 6; ++i) {
         if (b->aux[i]) cudaStreamDestroy(b->aux[i]);
         if (b->join[i]) cudaEventDestroy(b->join[i]);
     }
@@ -223,33 +223,43 @@ static cudaError_t run_persistent(cumc_batch *b, int count) {
 }
 
 // Every problem of up to 16 x 254 cells on a cluster of its own, one cell per
-// thread (tube_kernel.cuh): the fewest CTAs that hold it, a power of two, and
-// while the whole batch leaves half the SMs idle twice as many (up to 8, at
-// least 16 cells each), since a CTA with fewer warps runs a stage sooner.
-// Problems with the same cluster are neighbours in the launch order; each such
-// class is one launch on a stream of its own, the largest first.  What does not
-// fit goes to the persistent kernel.
+// thread (tube_kernel.cuh): the fewest CTAs that hold it, a power of two.  CTAs
+// of 254 cells keep the most cells in flight; a batch whose CTAs are all
+// resident at once (two an SM) waits for its largest problems, and those run
+// sooner on CTAs of 126 cells (PPM FP64, wide and narrow: 64 problems of 128 to
+// 2048 cells, 1.6 CTAs an SM, 14.0 and 10.9 ms; 128, 3.3 an SM, 14.8 and 15.4;
+// 512 of 128 to 4096, 22 an SM, 163 and 179).  A batch that leaves half the
+// SMs idle takes twice as many CTAs (up to 8, at least 16 cells each): a CTA
+// with fewer warps runs a stage sooner.  Problems with the same cluster are
+// neighbours in the launch order; each such class is one launch on a stream of
+// its own, the largest first.  What does not fit goes to the persistent kernel.
 static cudaError_t run_tubes(cumc_batch *b) {
-    const int np = b->nprob;
-    auto ctas = [&](int n) {
+    const int np = b->nprob, most = 16 * 254;
+    int big = 0;  // problems beyond 16 CTAs
+    while (big < np && b->sorted_n[big] > most) ++big;
+    auto ctas = [&](int n, int cells) {
         int c = 1;
-        while (c < 16 && (n + c - 1) / c > TUBE_MOST_CELLS) c *= 2;
+        while (c < 16 && (n + c - 1) / c > cells) c *= 2;
         return c;
     };
-    int big = 0;  // problems beyond 16 CTAs
-    while (big < np && b->sorted_n[big] > 16 * TUBE_MOST_CELLS) ++big;
     long long total = 0;
-    for (int p = big; p < np; ++p) total += ctas(b->sorted_n[p]);
+    for (int p = big; p < np; ++p) total += ctas(b->sorted_n[p], 254);
+    const bool narrow = total <= 2LL * b->sm_count;
+    auto wide_of = [&](int n) { return !narrow || n > 16 * 126; };
+    if (narrow) {
+        total = 0;
+        for (int p = big; p < np; ++p) total += ctas(b->sorted_n[p], wide_of(b->sorted_n[p]) ? 254 : 126);
+    }
     int wider = 1;
     while (wider < 8 && 2 * wider * total <= b->sm_count) wider *= 2;
     auto size_of = [&](int n) {
-        int c = ctas(n);
+        int c = ctas(n, wide_of(n) ? 254 : 126);
         for (int w = wider; w > 1 && c < 8 && n / (2 * c) >= 16; w /= 2) c *= 2;
         return c;
     };
     if (!b->fork) {
         cudaError_t e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
-        for (int i = 0; i < 4 && e == cudaSuccess; ++i) {
+        for (int i = 0; i < 6 && e == cudaSuccess; ++i) {
             e = cudaStreamCreateWithFlags(&b->aux[i], cudaStreamNonBlocking);
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join[i], cudaEventDisableTiming);
         }
@@ -260,20 +270,21 @@ static cudaError_t run_tubes(cumc_batch *b) {
     for (int p = big; p < np && e == cudaSuccess;) {
         const int size = size_of(b->sorted_n[p]);
         int q = p;
-        while (q < np && size_of(b->sorted_n[q]) == size) ++q;
-        cudaStream_t st = used < 4 ? b->aux[used] : b->stream;
-        if (used < 4) e = cudaStreamWaitEvent(st, b->fork, 0);
+        const bool wide = wide_of(b->sorted_n[p]);
+        while (q < np && size_of(b->sorted_n[q]) == size && wide_of(b->sorted_n[q]) == wide) ++q;
+        cudaStream_t st = used < 6 ? b->aux[used] : b->stream;
+        if (used < 6) e = cudaStreamWaitEvent(st, b->fork, 0);
         if (e == cudaSuccess)
-            e = b->precision == CUMC_FP32 ? launch_tube_fp32(b->d, b->recon, b->riemann, p, q - p, size, st)
-                                          : launch_tube_fp64(b->d, b->recon, b->riemann, p, q - p, size, st);
+            e = b->precision == CUMC_FP32 ? launch_tube_fp32(b->d, b->recon, b->riemann, p, q - p, size, wide, st)
+                                          : launch_tube_fp64(b->d, b->recon, b->riemann, p, q - p, size, wide, st);
         if (e != cudaSuccess && size == 16 && p == big) {
-            cudaGetLastError();  // no room for a 16-CTA cluster
+            cudaGetLastError();  // no room for a 16-CTA cluster: these are the largest, a prefix
             big = p = q;
             e = cudaSuccess;
             continue;
         }
         b->launches++;
-        if (used < 4 && e == cudaSuccess) {
+        if (used < 6 && e == cudaSuccess) {
             e = cudaEventRecord(b->join[used], st);
             ++used;
         }

@@ -542,10 +542,9 @@ static cudaError_t launch_batch_t(const BatchDev &b, int rec, int rs, int cluste
 }
 
 // tube_kernel.cuh: problems first .. first + count - 1 of b.order, one cluster of
-// `size` CTAs each
-constexpr int TUBE_MOST_CELLS = 254;  // of one CTA
-cudaError_t launch_tube_fp64(const BatchDev &b, int rec, int rs, int first, int count, int size, cudaStream_t s);
-cudaError_t launch_tube_fp32(const BatchDev &b, int rec, int rs, int first, int count, int size, cudaStream_t s);
+// `size` CTAs each, of 254 cells (wide) or 126
+cudaError_t launch_tube_fp64(const BatchDev &b, int rec, int rs, int first, int count, int size, int wide, cudaStream_t s);
+cudaError_t launch_tube_fp32(const BatchDev &b, int rec, int rs, int first, int count, int size, int wide, cudaStream_t s);
 
 // clusters <= 0: as many clusters of cluster_size CTAs as fit on the device
 cudaError_t launch_batch_fp64(const BatchDev &b, int rec, int rs, int clusters, int cluster_size, cudaStream_t s);

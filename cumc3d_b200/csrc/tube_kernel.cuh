@@ -20,10 +20,10 @@
 
 namespace cumc {
 
-constexpr int TUBE_THREADS = 256;
-static_assert(TUBE_MOST_CELLS == TUBE_THREADS - 2, "one more cell reconstructed on each side");
-constexpr int TUBE_ROW = 264;                 // padded row of one quantity
 constexpr int TUBE_MAX_CTAS = 16;
+// CTAs of NT threads hold NT - 2 cells (one more is reconstructed on each side);
+// a row of one quantity has their 3 + 3 ghosts and two spare
+constexpr int tube_row(int nt) { return nt + 8; }
 
 // rows of shared memory, in doubles
 enum : int {
@@ -35,11 +35,14 @@ enum : int {
     TS_E = TS_O + 8, TS_U4, TS_BY1, TS_BZ1, TS_BY0, TS_BZ0, TS_DX,
     TS_ROWS
 };
-constexpr int TUBE_SMEM = TS_ROWS * TUBE_ROW * 8;
+constexpr int tube_smem(int nt) { return TS_ROWS * tube_row(nt) * 8; }
 
-// problems first .. first + gridDim.x / clusterDim.x - 1 of b.order, one each
-template <class T, int REC, int RS>
-__global__ void __launch_bounds__(TUBE_THREADS, 2) k_tube(const BatchDev b, int first) {
+// problems first .. first + gridDim.x / clusterDim.x - 1 of b.order, one each.
+// NT = 256: 128 registers, two CTAs an SM (the most cells in flight); 128: twice
+// the registers, no spills, and half the warps in each other's way.
+template <class T, int REC, int RS, int NT>
+__global__ void __launch_bounds__(NT, 2) k_tube(const BatchDev b, int first) {
+    constexpr int TUBE_THREADS = NT, TUBE_ROW = tube_row(NT);
     extern __shared__ __align__(16) double sm[];
     __shared__ double part_dt[2][TUBE_MAX_CTAS];
     __shared__ int part_bad[2][TUBE_MAX_CTAS];
@@ -355,16 +358,16 @@ __global__ void __launch_bounds__(TUBE_THREADS, 2) k_tube(const BatchDev b, int 
     gbar();  // no CTA leaves while another may still write to it
 }
 
-template <class T, int REC, int RS>
+template <class T, int REC, int RS, int NT>
 static cudaError_t launch_tube_one(const BatchDev &b, int first, int count, int size, cudaStream_t s) {
-    cudaError_t e = cudaFuncSetAttribute(k_tube<T, REC, RS>, cudaFuncAttributeMaxDynamicSharedMemorySize, TUBE_SMEM);
+    cudaError_t e = cudaFuncSetAttribute(k_tube<T, REC, RS, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, tube_smem(NT));
     if (e == cudaSuccess && size > 8)
-        e = cudaFuncSetAttribute(k_tube<T, REC, RS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        e = cudaFuncSetAttribute(k_tube<T, REC, RS, NT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(count * size);
-    cfg.blockDim = dim3(TUBE_THREADS);
-    cfg.dynamicSmemBytes = TUBE_SMEM;
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = tube_smem(NT);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -373,17 +376,17 @@ static cudaError_t launch_tube_one(const BatchDev &b, int first, int count, int 
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_tube<T, REC, RS>, b, first);
+    return cudaLaunchKernelEx(&cfg, k_tube<T, REC, RS, NT>, b, first);
 }
 
 template <class T>
-static cudaError_t launch_tube_t(const BatchDev &b, int rec, int rs, int first, int count, int size, cudaStream_t s) {
+static cudaError_t launch_tube_t(const BatchDev &b, int rec, int rs, int first, int count, int size, int wide, cudaStream_t s) {
 #define CUMC_TUBE_RS(R)                                                                    \
     switch (rs) {                                                                          \
-        case RS_LF: return launch_tube_one<T, R, RS_LF>(b, first, count, size, s);         \
-        case RS_HLL: return launch_tube_one<T, R, RS_HLL>(b, first, count, size, s);       \
-        case RS_HLLC: return launch_tube_one<T, R, RS_HLLC>(b, first, count, size, s);     \
-        default: return launch_tube_one<T, R, RS_HLLD>(b, first, count, size, s);          \
+        case RS_LF: return wide ? launch_tube_one<T, R, RS_LF, 256>(b, first, count, size, s) : launch_tube_one<T, R, RS_LF, 128>(b, first, count, size, s); \
+        case RS_HLL: return wide ? launch_tube_one<T, R, RS_HLL, 256>(b, first, count, size, s) : launch_tube_one<T, R, RS_HLL, 128>(b, first, count, size, s); \
+        case RS_HLLC: return wide ? launch_tube_one<T, R, RS_HLLC, 256>(b, first, count, size, s) : launch_tube_one<T, R, RS_HLLC, 128>(b, first, count, size, s); \
+        default: return wide ? launch_tube_one<T, R, RS_HLLD, 256>(b, first, count, size, s) : launch_tube_one<T, R, RS_HLLD, 128>(b, first, count, size, s); \
     }
     switch (rec) {
         case REC_TVD_MM: CUMC_TUBE_RS(REC_TVD_MM);
