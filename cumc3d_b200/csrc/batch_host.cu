@@ -32,6 +32,9 @@ struct cumc_batch {
     cudaEvent_t fork = nullptr, join[6] = {};
 };
 
+// P 0..4, BX, BY1, BZ1, EPS (read back), BY0, BZ0
+constexpr int IO_ROWS = 11, IO_OUT = 9;
+
 static std::string g_batch_err;
 
 static int bfail(cumc_batch *b, int code, const std::string &m) {
@@ -109,10 +112,14 @@ int cumc_batch_create(const cumc_batch_config *cfg, cumc_batch **out) {
         return p;
     };
     const size_t nb = (size_t)tot * sizeof(double);
-    for (int i = 0; i < 5; ++i) { d.P[i] = (double *)A(nb); d.U[i] = (double *)A(nb); d.O[i] = (double *)A(nb); d.F[i] = (double *)A(nb); }
-    d.EPS = (double *)A(nb); d.CS = (double *)A(nb);
+    // the rows that cross to and from the host, one block: a problem's share of
+    // all of them is one 2D copy
+    double *io = (double *)A(nb * IO_ROWS);
+    double **io_rows[IO_ROWS] = {&d.P[0], &d.P[1], &d.P[2], &d.P[3], &d.P[4], &d.BX, &d.BY1, &d.BZ1, &d.EPS, &d.BY0, &d.BZ0};
+    for (int i = 0; i < IO_ROWS; ++i) *io_rows[i] = io ? io + (size_t)i * tot : nullptr;
+    for (int i = 0; i < 5; ++i) { d.U[i] = (double *)A(nb); d.O[i] = (double *)A(nb); d.F[i] = (double *)A(nb); }
+    d.CS = (double *)A(nb);
     for (int i = 0; i < 3; ++i) d.BC[i] = (double *)A(nb);
-    d.BX = (double *)A(nb); d.BY1 = (double *)A(nb); d.BZ1 = (double *)A(nb); d.BY0 = (double *)A(nb); d.BZ0 = (double *)A(nb);
     d.UBX = (double *)A(nb); d.UBXb = (double *)A(nb); d.UBY1 = (double *)A(nb); d.UBZ1 = (double *)A(nb); d.UBY0 = (double *)A(nb); d.UBZ0 = (double *)A(nb);
     d.OBX = (double *)A(nb); d.OBY1 = (double *)A(nb); d.OBZ1 = (double *)A(nb); d.OBY0 = (double *)A(nb); d.OBZ0 = (double *)A(nb);
     for (int i = 0; i < 7; ++i) { d.QL[i] = A(nb); d.QR[i] = A(nb); }
@@ -161,19 +168,18 @@ int cumc_batch_set_state(cumc_batch *b, int p, const double *prim, const double 
     const int n = b->n[p], NX = n + 6;
     auto ip = [&](int v, int j, int k, int l) { return (size_t)v + 8 * ((size_t)(j + 2) + NX * ((size_t)(k + 2) + 7 * (size_t)(l + 2))); };
     auto ie = [&](int j, int k, int l) { return (size_t)(j + 2) + NX * ((size_t)(k + 2) + 7 * (size_t)(l + 2)); };
-    std::vector<double> row((size_t)NX);
-    const long long o = b->off[p];
-    auto up = [&](double *dst, int v, int k, int l) {
-        for (int j = -2; j <= n + 3; ++j) row[j + 2] = prim[ip(v, j, k, l)];
-        return cudaMemcpyAsync(dst + o, row.data(), NX * sizeof(double), cudaMemcpyHostToDevice, b->stream) == cudaSuccess;
-    };
-    bool ok = true;
-    for (int v = 0; v < 5; ++v) ok = ok && up(b->d.P[v], v, 1, 1);
-    ok = ok && up(b->d.BX, 5, 1, 1) && up(b->d.BY1, 6, 1, 1) && up(b->d.BZ1, 7, 1, 1);
-    ok = ok && up(b->d.BY0, 6, 0, 1) && up(b->d.BZ0, 7, 1, 0);
-    for (int j = -2; j <= n + 3; ++j) row[j + 2] = eps[ie(j, 1, 1)];
-    ok = ok && cudaMemcpyAsync(b->d.EPS + o, row.data(), NX * sizeof(double), cudaMemcpyHostToDevice, b->stream) == cudaSuccess;
-    ok = ok && cudaStreamSynchronize(b->stream) == cudaSuccess;
+    // rows in the order of the device block
+    struct Src { int v, k, l; };
+    const Src src[IO_ROWS] = {{0, 1, 1}, {1, 1, 1}, {2, 1, 1}, {3, 1, 1}, {4, 1, 1}, {5, 1, 1},
+                              {6, 1, 1}, {7, 1, 1}, {-1, 1, 1}, {6, 0, 1}, {7, 1, 0}};
+    std::vector<double> rows((size_t)NX * IO_ROWS);
+    for (int r = 0; r < IO_ROWS; ++r)
+        for (int j = -2; j <= n + 3; ++j)
+            rows[(size_t)r * NX + j + 2] = src[r].v < 0 ? eps[ie(j, 1, 1)] : prim[ip(src[r].v, j, src[r].k, src[r].l)];
+    const bool ok = cudaMemcpy2DAsync(b->d.P[0] + b->off[p], (size_t)b->total * sizeof(double), rows.data(),
+                                      NX * sizeof(double), NX * sizeof(double), IO_ROWS, cudaMemcpyHostToDevice,
+                                      b->stream) == cudaSuccess &&
+                    cudaStreamSynchronize(b->stream) == cudaSuccess;
     return ok ? CUMC_OK : bfail(b, CUMC_ECUDA, "state upload failed");
 }
 
@@ -181,15 +187,14 @@ int cumc_batch_get_state(cumc_batch *b, int p, double *prim_row, double *eps_row
     if (!b || !prim_row || !eps_row || p < 0 || p >= b->nprob) return bfail(b, CUMC_EINVAL, "bad argument");
     const int n = b->n[p], NX = n + 6;
     const long long o = b->off[p];
-    std::vector<double> row(NX);
-    double *src[8] = {b->d.P[0], b->d.P[1], b->d.P[2], b->d.P[3], b->d.P[4], b->d.BX, b->d.BY1, b->d.BZ1};
-    for (int v = 0; v < 8; ++v) {
-        if (cudaMemcpy(row.data(), src[v] + o, NX * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess)
-            return bfail(b, CUMC_ECUDA, "download failed");
-        for (int j = 0; j < NX; ++j) prim_row[(size_t)j * 8 + v] = row[j];
-    }
-    if (cudaMemcpy(eps_row, b->d.EPS + o, NX * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess)
+    std::vector<double> rows((size_t)NX * IO_OUT);
+    if (cudaMemcpy2DAsync(rows.data(), NX * sizeof(double), b->d.P[0] + o, (size_t)b->total * sizeof(double),
+                          NX * sizeof(double), IO_OUT, cudaMemcpyDeviceToHost, b->stream) != cudaSuccess ||
+        cudaStreamSynchronize(b->stream) != cudaSuccess)
         return bfail(b, CUMC_ECUDA, "download failed");
+    for (int v = 0; v < 8; ++v)
+        for (int j = 0; j < NX; ++j) prim_row[(size_t)j * 8 + v] = rows[(size_t)v * NX + j];
+    memcpy(eps_row, &rows[(size_t)8 * NX], NX * sizeof(double));
     return CUMC_OK;
 }
 

@@ -1035,15 +1035,22 @@ __global__ void k_divb(const Dev d, unsigned long long *out) {
 }
 
 // Fortran layout prim(8, j, k, l) <-> structure of arrays (8 x N3)
-__global__ void k_aos_to_soa(const Dev d, const double *__restrict__ aos, int nv, double *const *dst) {
+struct Rows8 {
+    double *a[8];
+};
+__global__ void k_aos_to_soa(const Dev d, const double *__restrict__ aos, int nv, const Rows8 dst) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= d.N3) return;
-    for (int v = 0; v < nv; ++v) dst[v][c] = aos[(size_t)c * nv + v];
+    #pragma unroll
+    for (int v = 0; v < 8; ++v)
+        if (v < nv) dst.a[v][c] = aos[(size_t)c * nv + v];
 }
-__global__ void k_soa_to_aos(const Dev d, double *__restrict__ aos, int nv, const double *const *src) {
+__global__ void k_soa_to_aos(const Dev d, double *__restrict__ aos, int nv, const Rows8 src) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= d.N3) return;
-    for (int v = 0; v < nv; ++v) aos[(size_t)c * nv + v] = src[v][c];
+    #pragma unroll
+    for (int v = 0; v < 8; ++v)
+        if (v < nv) aos[(size_t)c * nv + v] = src.a[v][c];
 }
 
 // exhaustive-style check of div3 against the IEEE division: a counter-based
@@ -1174,7 +1181,7 @@ struct cumc_handle {
     Scalars *S_host = nullptr;  // pinned mirror
     unsigned long long *divb_dev = nullptr;
     double *stage_aos = nullptr;   // 8*N3 doubles (the u_old block doubles as transpose staging)
-    double **ptr_tab = nullptr;    // device table of 8 array pointers for the transposes
+    size_t cell_stride = 0;        // between the arrays of the cell B and c_s block
     int prof_class = -1;           // >= 0 while cumc_profile_step is recording
     cudaEvent_t ev[2] = {nullptr, nullptr};
     double prof_ms[16];
@@ -1733,22 +1740,28 @@ int cumc_create(const cumc_config *cfg, cumc_handle **out) {
     }
     bool ok = true;
     auto A = [&](double *&p, size_t n) { p = dalloc(h, n); ok = ok && p; };
-    for (int i = 0; i < 8; ++i) { A(d.P[i], N3); A(d.U[i], N3); }
+    for (int i = 0; i < 8; ++i) A(d.P[i], N3);
+    {
+        double *blk = nullptr;  // one block: cumc_set_state clears it with one call
+        A(blk, (size_t)8 * N3);
+        for (int i = 0; i < 8; ++i) d.U[i] = blk ? blk + (size_t)i * N3 : nullptr;
+    }
     {
         double *blk = dalloc(h, (size_t)8 * N3);
         ok = ok && blk;
         for (int i = 0; i < 8; ++i) d.U0[i] = blk ? blk + (size_t)i * N3 : nullptr;
         h->stage_aos = blk;
     }
-    {
-        void *t = nullptr;
-        ok = ok && cudaMalloc(&t, 8 * sizeof(double *)) == cudaSuccess;
-        if (t) h->allocs.push_back(t);
-        h->ptr_tab = (double **)t;
-    }
     ok = ok && cudaEventCreate(&h->ev[0]) == cudaSuccess && cudaEventCreate(&h->ev[1]) == cudaSuccess;
-    A(d.EPS, N3); A(d.CS, N3);
-    for (int i = 0; i < 3; ++i) { A(d.BC[i], N3); A(d.EC[i], N3); }
+    A(d.EPS, N3);
+    {
+        double *blk = nullptr;  // likewise; 256-byte steps (tensor maps start on the arrays)
+        h->cell_stride = ((size_t)N3 + 31) & ~(size_t)31;
+        A(blk, 4 * h->cell_stride);
+        for (int i = 0; i < 3; ++i) d.BC[i] = blk ? blk + i * h->cell_stride : nullptr;
+        d.CS = blk ? blk + 3 * h->cell_stride : nullptr;
+    }
+    for (int i = 0; i < 3; ++i) A(d.EC[i], N3);
     for (int i = 0; i < 5; ++i) {
         A(d.FX[i], N3);
         if (d.n_dim > 1) A(d.FY[i], N3); else d.FY[i] = d.FX[i];
@@ -1886,16 +1899,14 @@ int cumc_set_state(cumc_handle *h, const double *prim, const double *eps) {
     const size_t n3 = (size_t)d.N3;
     // one copy of the Fortran-layout buffer, transposed on the device
     CK(cudaMemcpyAsync(h->stage_aos, prim, 8 * n3 * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->ptr_tab, d.P, 8 * sizeof(double *), cudaMemcpyHostToDevice, h->stream));
-    k_aos_to_soa<<<(d.N3 + 255) / 256, 256, 0, h->stream>>>(d, h->stage_aos, 8, h->ptr_tab);
+    Rows8 rows;
+    for (int v = 0; v < 8; ++v) rows.a[v] = d.P[v];
+    k_aos_to_soa<<<(d.N3 + 255) / 256, 256, 0, h->stream>>>(d, h->stage_aos, 8, rows);
     h->launches++;
     CK(cudaMemcpyAsync(d.EPS, eps, n3 * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-    for (int v = 0; v < 8; ++v) {
-        CK(cudaMemsetAsync(d.U[v], 0, n3 * sizeof(double), h->stream));
-        CK(cudaMemsetAsync(d.U0[v], 0, n3 * sizeof(double), h->stream));
-    }
-    for (int i = 0; i < 3; ++i) CK(cudaMemsetAsync(d.BC[i], 0, n3 * sizeof(double), h->stream));
-    CK(cudaMemsetAsync(d.CS, 0, n3 * sizeof(double), h->stream));
+    // (u_old, the transposes' staging, is written by stage 1 before any use)
+    CK(cudaMemsetAsync(d.U[0], 0, 8 * n3 * sizeof(double), h->stream));
+    CK(cudaMemsetAsync(d.BC[0], 0, 4 * h->cell_stride * sizeof(double), h->stream));
     CK(cudaStreamSynchronize(h->stream));
     h->have_state = true;
     h->initialised = false;
@@ -1905,9 +1916,10 @@ int cumc_set_state(cumc_handle *h, const double *prim, const double *eps) {
 static int download_aos(cumc_handle *h, double *const *src_host, int nv, double *out) {
     const Dev &d = h->d;
     const size_t n3 = (size_t)d.N3;
-    CK(cudaMemcpyAsync(h->ptr_tab, src_host, nv * sizeof(double *), cudaMemcpyHostToDevice, h->stream));
+    Rows8 rows;
+    for (int v = 0; v < 8; ++v) rows.a[v] = v < nv ? src_host[v] : nullptr;
     // the u_old block is free between steps; it only holds stage-1 backups
-    k_soa_to_aos<<<(d.N3 + 255) / 256, 256, 0, h->stream>>>(d, h->stage_aos, nv, h->ptr_tab);
+    k_soa_to_aos<<<(d.N3 + 255) / 256, 256, 0, h->stream>>>(d, h->stage_aos, nv, rows);
     h->launches++;
     CK(cudaMemcpyAsync(out, h->stage_aos, nv * n3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
