@@ -2321,7 +2321,7 @@ int cumc_poisson_setup(cumc_handle *h, double rho_atm, double omega) {
         s.ajm1 = (double *)A(px * sizeof(double));
         s.bkp1 = (double *)A(py * sizeof(double));
         s.bkm1 = (double *)A(py * sizeof(double));
-        s.err = (unsigned long long *)A(sizeof(unsigned long long));
+        s.err = (unsigned long long *)A(2 * sizeof(unsigned long long));
         s.state = (int *)A(4 * sizeof(int));
         s.tol = (double *)A(sizeof(double));
         s.err_last = (double *)A(sizeof(double));
@@ -2386,24 +2386,29 @@ int cumc_poisson_solve(cumc_handle *h, int max_iter, double tol, int *iters_out,
     CK(cudaMemcpyAsync(s.state + 2, lim, sizeof(int), cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemcpyAsync(s.tol, &tol, sizeof(double), cudaMemcpyHostToDevice, h->stream));
     launch_sor_reset(s, h->stream);
+    constexpr int PER_GRAPH = 16;  // even: a captured iteration keeps its parity
     if (!h->sor_exec) {
         CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        launch_sor_iteration(s, h->stream);
+        for (int i = 0; i < PER_GRAPH; ++i) launch_sor_iteration(s, 2 + i, h->stream);
         CK(cudaStreamEndCapture(h->stream, &h->sor_graph));
         CK(cudaGraphInstantiate(&h->sor_exec, h->sor_graph, 0));
     }
-    // replay in chunks; once the device marks the loop finished, the
-    // remaining launches of a chunk return at once
-    int st[3] = {0, 0, 0};
-    while (true) {
+    launch_sor_iteration(s, 1, h->stream);
+    h->launches += 3;
+    // replay up to 64 iterations at a time; once the device marks the loop
+    // finished (tolerance or limit), the launches that remain return at once
+    int st[3] = {1, 0, 0};
+    while (st[1] == 0 && st[0] < max_iter) {
         const int left = max_iter - st[0];
-        const int chunk = left < 32 ? left : 32;
-        for (int i = 0; i < chunk; ++i) CK(cudaGraphLaunch(h->sor_exec, h->stream));
-        h->launches += 3LL * chunk;
+        const int graphs = left > 3 * PER_GRAPH ? 4 : (left + PER_GRAPH - 1) / PER_GRAPH;
+        for (int i = 0; i < graphs; ++i) CK(cudaGraphLaunch(h->sor_exec, h->stream));
+        h->launches += 2LL * PER_GRAPH * graphs;
         CK(cudaMemcpyAsync(st, s.state, 3 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));
-        if (st[1] != 0) break;
     }
+    launch_sor_ghosts(s, 1, h->stream);
+    h->launches++;
+    CK(cudaMemcpyAsync(st, s.state, 3 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     double e = 0.0;
     CK(cudaMemcpyAsync(&e, s.err_last, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
@@ -2821,28 +2826,20 @@ int cumc_collapsar_get(cumc_handle *h, double *m_bh, double *r_sh) {
 static int poisson_copy(cumc_handle *h, double *out, const double *in) {
     if (!h) return fail(h, CUMC_EINVAL, "null handle");
     if (!h->sor_ready) return fail(h, CUMC_ENOTREADY, "cumc_poisson_setup first");
-    SorDev &s = h->sor;
-    const long long px = s.nx + 2, py = (long long)(s.nx + 2) * (s.ny + 2);
-    const long long half = (long long)s.hx * (s.ny + 2) * (s.nz + 2);
-    std::vector<double> part[2];
-    for (int c = 0; c < 2; ++c) part[c].assign(half, 0.0);
-    if (out) {
-        for (int c = 0; c < 2; ++c)
-            CK(cudaMemcpyAsync(part[c].data(), s.phi[c], half * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
-    }
-    for (int l = 0; l <= s.nz + 1; ++l)
-        for (int k = 0; k <= s.ny + 1; ++k)
-            for (int j = 0; j <= s.nx + 1; ++j) {
-                const long long n = j + px * k + py * l, q = sor_index(s, j, k, l);
-                if (out) out[n] = part[(j + k + l) & 1][q];
-                else part[(j + k + l) & 1][q] = in[n];
-            }
+    const SorDev &s = h->sor;
+    // the natural order passes through the transposes' staging (8 padded cells'
+    // worth, more than the potential); the colours are split and joined there
+    const size_t bytes = (size_t)(s.nx + 2) * (s.ny + 2) * (s.nz + 2) * sizeof(double);
     if (in) {
-        for (int c = 0; c < 2; ++c)
-            CK(cudaMemcpyAsync(s.phi[c], part[c].data(), half * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
+        CK(cudaMemcpyAsync(h->stage_aos, in, bytes, cudaMemcpyHostToDevice, h->stream));
+        launch_sor_order(s, h->stage_aos, 1, h->stream);
+    } else {
+        launch_sor_order(s, h->stage_aos, 0, h->stream);
+        CK(cudaMemcpyAsync(out, h->stage_aos, bytes, cudaMemcpyDeviceToHost, h->stream));
     }
+    h->launches++;
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(h->stream));
     return CUMC_OK;
 }
 int cumc_poisson_get(cumc_handle *h, double *phi) {

@@ -25,8 +25,8 @@ struct SorDev {
     const double *ajp1, *ajm1;                  // per j = 0..nx+1
     const double *bkp1, *bkm1;                  // per (j, k): j + (nx + 2) * k
     double omega;
-    // loop state on the device: the iteration's max |dphi / phi_old| (bit
-    // pattern of a non-negative double), [0] iterations taken, [1] 0 running /
+    // loop state on the device: max |dphi / phi_old| of the odd and the even
+    // iterations (bit pattern of a non-negative double), [0] iterations taken, [1] 0 running /
     // 1 converged / 2 iteration limit, [2] the limit; the tolerance; the last
     // iteration's error
     unsigned long long *err;
@@ -43,7 +43,9 @@ __host__ __device__ inline long long sor_index(const SorDev &s, int j, int k, in
 void sor_coefficients(int nx, int ny, int nz, const double *x, const double *y, const double *z, double *ajp1,
                       double *ajm1, double *bkp1, double *bkm1, double *clp1, double *clm1, double *epsc);
 void launch_sor_source(const SorDev &s, const double *rho, int NX, int NY, double rho_atm, cudaStream_t st);
-void launch_sor_iteration(const SorDev &s, cudaStream_t st);
+void launch_sor_iteration(const SorDev &s, int it, cudaStream_t st);
+void launch_sor_ghosts(const SorDev &s, int end, cudaStream_t st);
+void launch_sor_order(const SorDev &s, double *nat, int split, cudaStream_t st);
 void launch_sor_reset(const SorDev &s, cudaStream_t st);
 
 }  // namespace cumc
