@@ -1776,7 +1776,8 @@ int cumc_create(const cumc_config *cfg, cumc_handle **out) {
         d.QR[i] = b;
     }
     A(d.EX, N3); A(d.EY, N3); A(d.EZ, N3);
-    if (cfg->precision == CUMC_FP64 && cfg->riemann == CUMC_RS_HLLD) {
+    // (up to 131072 cells the list's launch costs a stage more than it saves)
+    if ((long long)nx * ny * nz > 131072 && cfg->precision == CUMC_FP64 && cfg->riemann == CUMC_RS_HLLD) {
         // the list of deferred faces: one cell in 4 (34 B a cell, 5% of a
         // handle), at least 256; the spherical torus fills 0.07 a cell
         d.fix_cap = (unsigned)(N3 / 4 > 256 ? N3 / 4 : 256);

@@ -101,14 +101,14 @@ __device__ __forceinline__ void store_face(const Dev &d, int ci, const T *fo) {
 // about one face in a hundred where fields decay towards zero (products
 // between 1e-323 and 1e-271), but spread so that the plain form inside this
 // kernel ran in most warps (spherical torus 124 x 44 x 128, the three sweeps
-// of a step: 1.45 ms that way, 0.87 with the list).  A full list falls back to
-// the plain form here.
+// of a step: 1.45 ms that way, 0.87 with the list).  Without a list
+// (small grids) or when it is full, the plain form runs here.
 template <class T, int DIR, int RS>
 __device__ __forceinline__ void solve_face(const Dev &d, int ci, const T *pl, const T *pr) {
     T fo[9];
     if constexpr (sizeof(T) == sizeof(double) && RS == RS_HLLD) {
         if (!hlld64<DIR>(pl, pr, d.gamma, fo)) {
-            const unsigned slot = atomicAdd(d.fix_n, 1u);
+            const unsigned slot = d.fix_n ? atomicAdd(d.fix_n, 1u) : d.fix_cap;  // no list on small grids
             double q[17];
 #pragma unroll
             for (int i = 1; i <= 8; ++i) {
