@@ -1,12 +1,11 @@
 // fast64.cuh -- the FP64 reconstruction and Riemann arithmetic without
 // branches in its divisions and square roots.
 //
-// The plain forms (mhd_device.cuh) divide with the IEEE operator, which the
-// compiler expands to a refinement, a range test and a call for each division:
-// every division ends a basic block, so two independent divisions never
-// overlap and the kernels wait out one dependency chain after the other (the
-// HLLD kernel ran its FP64 pipe 45% busy, 51% of issue slots, with 4 warps per
-// scheduler).  Here a quotient is a reciprocal refined from the hardware seed
+// The plain forms (mhd_device.cuh) divide with the IEEE operator, one guarded
+// division after the other, and the kernels waited out one dependency chain
+// after the other (128^3 blast, HLLD: FP64 pipe 45% busy, 51% of issue slots,
+// 4 warps per scheduler, 180 us a sweep; this form 63-68%, 101-109 us; WENO-Z
+// reconstruction 274 and 190 us).  Here a quotient is a reciprocal refined from the hardware seed
 // and one residual correction, straight-line code that the compiler
 // interleaves freely; one reciprocal serves every quotient over the same
 // divisor; and the operands' exponents are tested on the integer pipe, beside

@@ -101,7 +101,7 @@ __device__ __forceinline__ void store_face(const Dev &d, int ci, const T *fo) {
 // about one face in a hundred where fields decay towards zero (products
 // between 1e-323 and 1e-271), but spread so that the plain form inside this
 // kernel ran in most warps (spherical torus 124 x 44 x 128, the three sweeps
-// of a step: 1.45 ms that way, 0.87 with the list).  Without a list
+// of a step: 1.42 ms that way, 0.86 with the list).  Without a list
 // (small grids) or when it is full, the plain form runs here.
 template <class T, int DIR, int RS>
 __device__ __forceinline__ void solve_face(const Dev &d, int ci, const T *pl, const T *pr) {

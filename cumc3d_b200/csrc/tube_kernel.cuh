@@ -3,7 +3,7 @@
 //
 // batch_kernel.cuh keeps a problem's rows in global memory: every phase of a
 // stage waits for L2 round trips, three cluster barriers a stage, and a thread
-// works through two or more cells one after the other (11.7 us a stage for 800
+// works through two or more cells one after the other (13.9 us a stage for 800
 // cells on 8 CTAs).  Here a CTA holds up to 254 cells in shared memory, a cell
 // belongs to one thread for the whole run, and a stage has one cluster barrier:
 // each CTA reconstructs one cell and solves one face beyond its share instead of
