@@ -493,7 +493,12 @@ namespace cumc {
 // KIND: the recon_tile choice (1, 2, 4)
 template <class T, int DIR, int UNI, int CPT, int KIND>
 static void launch_recon_tile_c(const Dev &d, int rec, cudaStream_t s) {
-    const dim3 g = recon_tile_grid(d, DIR, CPT), b(32, 8, 1);
+    dim3 g = recon_tile_grid(d, DIR, CPT);
+    const dim3 b(32, 8, 1);
+    if (pack_x<T>(DIR, rec)) {
+        const XTail t = x_tail(d, CPT);
+        g = dim3(t.tiles + t.tails, 1, d.nz);
+    }
     // blocks per SM: FP64 WENO-Z unrolls to 250 registers where nothing bounds
     // it; 2 blocks (126 registers) and, as kind 4, 3 blocks (80, 152 B spilled)
     constexpr bool W = sizeof(T) == sizeof(double);

@@ -35,6 +35,36 @@ __host__ __device__ inline dim3 recon_tile_grid(const Dev &d, int dir, int cpt) 
     return dim3((d.nx + 31) / 32, (d.nz + 2 + nr - 1) / nr, d.ny);
 }
 
+// The x sweep's nx + 2 cells a row are seldom whole tiles (98 = 3 x 32 + 2): the
+// columns beyond the last whole tile, `rest` wide, go `rows` rows to a block, as
+// many as its threads and its shared memory hold, instead of 8 (x cpt) rows to a
+// block whose other lanes idle.  FP64 WENO-Z, ms a step before and now: 96 x 64 x 96
+// 1.199 and 1.163, 101 x 96 x 90 1.828 and 1.787, 160^3 7.68 and 7.54, 62 x 64 x 64,
+// whose rows are whole tiles, 0.568 and 0.567.
+struct XTail {
+    int full, rest, rows, tiles, tails;  // whole tiles a row, as above, blocks a plane of either kind
+};
+__host__ __device__ inline XTail x_tail(const Dev &d, int cpt) {
+    const int h = 2, nr = 8 * cpt;  // h: WENO-Z's halo
+    XTail t;
+    t.full = (d.nx + 2) / 32;
+    t.rest = (d.nx + 2) % 32;
+    t.rows = 1;
+    if (t.rest) {
+        const int a = 32 * nr / t.rest, b = nr * (32 + 2 * h) / (t.rest + 2 * h);
+        t.rows = a < b ? a : b;
+    }
+    t.tiles = t.full * ((d.ny + nr - 1) / nr);
+    t.tails = t.rest ? (d.ny + t.rows - 1) / t.rows : 0;
+    return t;
+}
+// Only FP64 WENO-Z, which is bound by the FP64 pipe the idle lanes keep busy: the
+// width known at run time cost FP32 more than that gave (192^3 7.69 -> 7.72), and
+// PPM won 0.6% (128^3) or lost as much (62 x 64 x 64).  Not with the learned flag,
+// whose warps are indexed by recon_tile_grid.
+template <class T>
+constexpr bool pack_x(int dir, int rec) { return dir == 0 && rec == REC_WENO && sizeof(T) == sizeof(double); }
+
 // The index of the warp of the staged reconstruction (learned_warps in
 // engine.cuh) with x-chunk bx, sweep cell c (DIR 1, 2) or row k (DIR 0) and
 // the remaining coordinate o (l for DIR 0 and 1, k for DIR 2).
@@ -100,9 +130,10 @@ __global__ void __launch_bounds__(256) k_learned_warps(const Dev d, int stage) {
 // SLOT elements, each SR rows of SX values; the stencil of the cell in row r,
 // lane tx sits at column tx + HO + m (x sweep) or row r + HO + m, column
 // tx + XO (y, z sweeps), m = -H..H.
-template <class T, int DIR, int REC, int UNI, int CPT, int LRN, int SX, int SLOT, int HO, int XO>
-__device__ __forceinline__ void recon_tile_cells(const Dev &d, const T *__restrict__ s, int bx, int by, int bz, int tx,
-                                                 int ty) {
+// PACK: x0, k0, the width and the rows of a block of the x sweep (x_tail).
+template <class T, int DIR, int REC, int UNI, int CPT, int LRN, int SX, int SLOT, int HO, int XO, bool PACK = false>
+__device__ __forceinline__ void recon_tile_cells(const Dev &d, const T *__restrict__ s, int bx, int by, int bz, int lane,
+                                                 int ty, int x0 = 0, int k0 = 0, int width = 32, int rows = 0) {
     constexpr int TX = 32, TY = 8;
     constexpr int H = (REC == REC_PPM || REC == REC_WENO) ? 2 : 1;
     constexpr int NR = TY * CPT;
@@ -112,10 +143,16 @@ __device__ __forceinline__ void recon_tile_cells(const Dev &d, const T *__restri
     const int st = (DIR == 0) ? 1 : (DIR == 1) ? d.NX : d.NX * d.NY;
 #pragma unroll
     for (int i = 0; i < CPT; ++i) {
-        const int r = ty + TY * i;  // row within the tile
+        int r = ty + TY * i, tx = lane;  // row and column within the tile
         int c, j, k, l, ns;
         bool valid;
-        if (DIR == 0) {
+        if (PACK) {
+            const int t = lane + TX * r;
+            r = t / width;
+            tx = t - r * width;
+            c = x0 + tx; j = c; k = k0 + r; l = bz + 1; ns = d.nx;
+            valid = r < rows && k <= d.ny;
+        } else if (DIR == 0) {
             c = c0 + tx; j = c; k = by * NR + r + 1; l = bz + 1; ns = d.nx;
             valid = c <= d.nx + 1 && k <= d.ny;
         } else if (DIR == 1) {
@@ -147,7 +184,7 @@ __device__ __forceinline__ void recon_tile_cells(const Dev &d, const T *__restri
         }
         // the stencil c-H .. c+H of variable v
         auto at = [&](int v, int m) -> T {
-            return (DIR == 0) ? s[v * SLOT + r * SX + tx + HO + m] : s[v * SLOT + (r + HO + m) * SX + tx + XO];
+            return (DIR == 0) ? s[v * SLOT + r * (PACK ? width + 2 * H : SX) + tx + HO + m] : s[v * SLOT + (r + HO + m) * SX + tx + XO];
         };
         auto put = [&](int v, T vm, T vp) {
             if (c <= ns) QL[v][ci] = vp;      // left state of face c
@@ -177,8 +214,36 @@ __global__ void __launch_bounds__(256, MINB) k_recon_tile(const Dev d, int stage
     constexpr int tb2 = (DIR == 2) ? 1 : 2;
 
     // ---- stage the tile ----
+    constexpr bool PACK = pack_x<T>(DIR, REC) && LRN == 0;
+    int x0 = 0, k0 = 1, width = TX, rows = NR;
+    if (PACK) {
+        const XTail t = x_tail(d, CPT);
+        const int b = blockIdx.x;
+        if (b < t.tiles) {
+            const int by = b / t.full;
+            x0 = (b - by * t.full) * TX;
+            k0 = by * NR + 1;
+        } else {
+            x0 = t.full * TX;
+            k0 = (b - t.tiles) * t.rows + 1;
+            width = t.rest;
+            rows = t.rows;
+        }
+        const int wx = width + 2 * H;
+        for (int idx = tid; idx < rows * wx; idx += TX * TY) {
+            const int sr = idx / wx, x = x0 - H + idx - sr * wx, y = k0 + sr;
+            if (y <= d.ny) {
+                const int ci = cidx(d, x, y, blockIdx.z + 1);
+#pragma unroll
+                for (int v = 0; v < 7; ++v) {
+                    const double *src = (v < 5) ? d.P[v] : d.BC[v == 5 ? tb1 : tb2];
+                    s[v * SR * SX + idx] = (T)__ldg(src + ci);
+                }
+            }
+        }
+    }
     const int c0 = (DIR == 0) ? blockIdx.x * TX : blockIdx.y * NR;  // first reconstructed cell
-    for (int idx = tid; idx < SR * SX; idx += TX * TY) {
+    for (int idx = tid; !PACK && idx < SR * SX; idx += TX * TY) {
         const int sr = idx / SX, sx = idx - sr * SX;
         int x, y, z;
         bool ok;
@@ -202,7 +267,8 @@ __global__ void __launch_bounds__(256, MINB) k_recon_tile(const Dev d, int stage
         }
     }
     __syncthreads();
-    recon_tile_cells<T, DIR, REC, UNI, CPT, LRN, SX, SR * SX, H, 0>(d, s, blockIdx.x, blockIdx.y, blockIdx.z, tx, ty);
+    recon_tile_cells<T, DIR, REC, UNI, CPT, LRN, SX, SR * SX, H, 0, PACK>(d, s, blockIdx.x, blockIdx.y, blockIdx.z, tx,
+                                                                                   ty, x0, k0, width, rows);
 }
 
 // ---------------------------------------------------------------------------
