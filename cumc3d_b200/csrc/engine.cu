@@ -86,6 +86,7 @@ struct GhostList {
     unsigned char var[13];   // parity index
 };
 constexpr int GHOST_GROUPS = 4;  // blockIdx.y: arrays 0-3, 4-7, 8-10, 11-12
+constexpr int GHOST_BZ = 10;     // P 7, the z face field
 
 // BOUNDARY (boundary.f90:5-770) and CUSTOM_BOUNDARY_X/Z (torus velocity clamps,
 // model/torus-cyn/src/custom.f90:146-208) in one pass over the ghost cells.  The
@@ -123,8 +124,11 @@ __global__ void __launch_bounds__(256) k_ghosts(const Dev d, const GhostList gl)
     } else {
         return;
     }
-    // a z side shared with a neighbouring slab is filled by the exchange
-    if ((l < 1 && d.zcut[0]) || (l > d.nz && d.zcut[1])) return;
+    // a z side shared with a neighbouring slab is filled by the exchange; at the
+    // seam of a ring that leaves out the normal field where the z fill does
+    // (halo_arrays), and its x and y ghosts are filled here as on any plane
+    const int cut = l < 1 ? d.zcut[0] : l > d.nz ? d.zcut[1] : 0;
+    if (cut && (cut == 1 || d.fixn)) return;
     const int c = cidx(d, j, k, l);
     int side[3], off[3];
     {
@@ -148,7 +152,7 @@ __global__ void __launch_bounds__(256) k_ghosts(const Dev d, const GhostList gl)
         const int m = first + q;
         v[q] = 0.0;
         moved[q] = false;
-        if (m >= last) continue;
+        if (m >= last || (cut && m != GHOST_BZ)) continue;
         int o = 0;
 #pragma unroll
         for (int x = 0; x < 3; ++x)
