@@ -2443,6 +2443,12 @@ struct DeviceGuard {
     ~DeviceGuard() { cudaSetDevice(dev); }
 };
 
+static void mark_seam(cumc_handle *h, int side) {
+    if (h->d.zcut[side] == 2) return;
+    h->d.zcut[side] = 2;
+    drop_graphs(h);
+}
+
 static int group_check(cumc_handle **hs, int n, bool *ring) {
     if (!hs || n < 2) return fail(nullptr, CUMC_EINVAL, "a group needs at least two slabs");
     for (int i = 0; i < n; ++i)
@@ -2465,8 +2471,8 @@ static int group_check(cumc_handle **hs, int n, bool *ring) {
     // the boundary rules (index-0 layer, clamps) and take only their fill data
     // from the neighbour
     if (*ring) {
-        hs[0]->d.zcut[0] = 2;
-        hs[n - 1]->d.zcut[1] = 2;
+        mark_seam(hs[0], 0);
+        mark_seam(hs[n - 1], 1);
     }
     return CUMC_OK;
 }
@@ -2655,7 +2661,7 @@ int cumc_slab_seam(cumc_handle *h, int side) {
     int rc = slab_side(h, CUMC_FILL_STATE, side);
     if (rc) return rc;
     if (h->initialised) return fail(h, CUMC_EINVAL, "mark the seam before cumc_slab_initial_begin");
-    h->d.zcut[side] = 2;
+    mark_seam(h, side);
     return CUMC_OK;
 }
 

@@ -46,3 +46,28 @@ def test_seam_planes_carry_the_undivided_ghosts(xy, sizes):
         s.rungekutta(dt)
     g.close()
     s.close()
+
+
+def test_captured_step_of_a_slab_follows_its_seam():
+    """A slab stepped by itself before it joins a ring keeps no step captured
+    with its old z sides."""
+    spec, prim, eps = _problem((0, 0, 0, 0))
+    out = []
+    for alone in (4, 0):
+        g = engine.SlabGroup(spec, (8, 7))
+        g.set_state(prim, eps)
+        if alone:
+            for s in g.slabs:
+                s.initial_update()
+                for _ in range(alone):
+                    s.rungekutta(1e-4)
+            g.set_state(prim, eps)
+        g.initial_update()
+        for s in g.slabs:
+            s.rungekutta(1e-3)
+        out.append([s.get_state() + (s.get_array(capi.ARR_CONS),) for s in g.slabs])
+        g.close()
+    inner = (slice(3, -3),) * 3
+    for a, b in zip(*out):
+        for x, y in zip(a, b):
+            assert np.array_equal(x[inner], y[inner])
