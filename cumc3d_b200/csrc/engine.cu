@@ -1619,6 +1619,16 @@ static int check_scalars(cumc_handle *h) {
     return CUMC_OK;
 }
 
+// Whether a handle's stage kernels are launched programmatically dependent.
+// 64^3 PPM 486 -> 467 us a step, 101 x 96 x 90 1379 -> 1354; below they cost
+// (24^3 128 -> 161, 64^2 104 -> 124).  Only where the launch before on the same
+// stream is the kernel a stage kernel depends on: not with concurrent sweeps,
+// whose join has several predecessors, and not for a slab, whose exchange puts
+// copies and waits on its neighbours' streams between two kernels twice a stage.
+static int programmatic(const Dev &d, bool concurrent) {
+    return d.N3 >= 200000 && !concurrent && !d.zcut[0] && !d.zcut[1] ? 1 : 0;
+}
+
 extern "C" {
 
 int cumc_create(const cumc_config *cfg, cumc_handle **out) {
@@ -1675,9 +1685,7 @@ int cumc_create(const cumc_config *cfg, cumc_handle **out) {
     d.tpb_recon = 256;
     d.tpb_riemann = 128;
     d.riemann_minb = 4;
-    // programmatic launches: 64^3 PPM 486 -> 467 us a step, 101 x 96 x 90 1379 ->
-    // 1354; below they cost (24^3 128 -> 161, 64^2 104 -> 124)
-    d.pdl = N3 >= 200000 ? 1 : 0;
+    d.pdl = programmatic(d, false);
     d.gamma = cfg->model.gamma; d.cfl = cfg->cfl;
     d.floor_kind = cfg->model.floor_kind; d.source_kind = cfg->model.source_kind; d.bc_kind = cfg->model.bc_kind;
     d.rho_floor = cfg->model.rho_floor; d.eps_floor = cfg->model.eps_floor; d.p_floor = cfg->model.p_floor;
@@ -2242,7 +2250,7 @@ int cumc_set_concurrent_sweeps(cumc_handle *h, int on) {
         for (int i = 0; i < 3; ++i) CK(cudaEventCreateWithFlags(&h->fev[i], cudaEventDisableTiming));
     }
     h->sweeps_concurrent = on != 0;
-    h->d.pdl = !on && h->d.N3 >= 200000 ? 1 : 0;  // a kernel after a join has several predecessors
+    h->d.pdl = programmatic(h->d, on != 0);
     // a captured step graph holds the old launch order
     drop_graphs(h);
     return CUMC_OK;

@@ -49,7 +49,7 @@ struct Dev {
     int tpb_recon, tpb_riemann;  // threads per block of the split flux kernels (autotuned)
     int riemann_minb;            // blocks/SM the Riemann kernel is compiled for (1, 4, 5, 6; 14, 15, 16:
                                  // the prefetching kernel at 4, 5, 6; autotuned)
-    int pdl;                     // launch() with programmatic dependence (not with concurrent sweeps)
+    int pdl;                     // launch() with programmatic dependence (not with concurrent sweeps or slabs)
     int recon_tile;              // 0: per-cell stencil loads; 1, 2: staged tiles, cells per thread (autotuned)
     int wuni[3];                 // 1: the axis's reconstruction weights are identical in every cell
     double wu[3][14];            // those weights (FP64 form)
