@@ -9,6 +9,7 @@
 
 #include "../../include/cumc3d_gpu.h"
 #include "batch_kernel.cuh"
+#include "tube_plan.h"
 #include "weights1d.cuh"
 
 using namespace cumc;
@@ -198,11 +199,12 @@ int cumc_batch_get_state(cumc_batch *b, int p, double *prim_row, double *eps_row
     return CUMC_OK;
 }
 
-// the first `count` problems (the largest) through the persistent kernel, whose
-// rows live in global memory: any size, any sharing
-static cudaError_t run_persistent(cumc_batch *b, int count) {
+// problems first .. first + count - 1 of the launch order through the persistent
+// kernel, whose rows live in global memory: any size, any sharing
+static cudaError_t run_persistent(cumc_batch *b, int first, int count) {
     if (cudaMemsetAsync(b->d.next, 0, sizeof(int), b->stream) != cudaSuccess) return cudaErrorUnknown;
     BatchDev d = b->d;
+    d.order += first;
     d.nprob = count;
     // sharing threshold: a batch no larger than the clusters that can be
     // resident at once (two 256-thread CTAs per SM) leaves SMs idle, so its
@@ -227,41 +229,9 @@ static cudaError_t run_persistent(cumc_batch *b, int count) {
     return e;
 }
 
-// Every problem of up to 16 x 254 cells on a cluster of its own, one cell per
-// thread (tube_kernel.cuh): the fewest CTAs that hold it, a power of two.  CTAs
-// of 254 cells keep the most cells in flight; a batch whose CTAs are all
-// resident at once (two an SM) waits for its largest problems, and those run
-// sooner on CTAs of 126 cells (PPM FP64, wide and narrow: 64 problems of 128 to
-// 2048 cells, 1.6 CTAs an SM, 14.0 and 10.9 ms; 128, 3.3 an SM, 14.8 and 15.4;
-// 512 of 128 to 4096, 22 an SM, 163 and 179).  A batch that leaves half the
-// SMs idle takes twice as many CTAs (up to 8, at least 16 cells each): a CTA
-// with fewer warps runs a stage sooner.  Problems with the same cluster are
-// neighbours in the launch order; each such class is one launch on a stream of
-// its own, the largest first.  What does not fit goes to the persistent kernel.
+// The batch as tube_plan.h lays it out, each class of clusters on a stream of its
+// own, the largest first.
 static cudaError_t run_tubes(cumc_batch *b) {
-    const int np = b->nprob, most = 16 * 254;
-    int big = 0;  // problems beyond 16 CTAs
-    while (big < np && b->sorted_n[big] > most) ++big;
-    auto ctas = [&](int n, int cells) {
-        int c = 1;
-        while (c < 16 && (n + c - 1) / c > cells) c *= 2;
-        return c;
-    };
-    long long total = 0;
-    for (int p = big; p < np; ++p) total += ctas(b->sorted_n[p], 254);
-    const bool narrow = total <= 2LL * b->sm_count;
-    auto wide_of = [&](int n) { return !narrow || n > 16 * 126; };
-    if (narrow) {
-        total = 0;
-        for (int p = big; p < np; ++p) total += ctas(b->sorted_n[p], wide_of(b->sorted_n[p]) ? 254 : 126);
-    }
-    int wider = 1;
-    while (wider < 8 && 2 * wider * total <= b->sm_count) wider *= 2;
-    auto size_of = [&](int n) {
-        int c = ctas(n, wide_of(n) ? 254 : 126);
-        for (int w = wider; w > 1 && c < 8 && n / (2 * c) >= 16; w /= 2) c *= 2;
-        return c;
-    };
     if (!b->fork) {
         cudaError_t e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
         for (int i = 0; i < 6 && e == cudaSuccess; ++i) {
@@ -271,31 +241,29 @@ static cudaError_t run_tubes(cumc_batch *b) {
         if (e != cudaSuccess) return e;
     }
     cudaError_t e = cudaEventRecord(b->fork, b->stream);
+    if (e != cudaSuccess) return e;
     int used = 0;
-    for (int p = big; p < np && e == cudaSuccess;) {
-        const int size = size_of(b->sorted_n[p]);
-        int q = p;
-        const bool wide = wide_of(b->sorted_n[p]);
-        while (q < np && size_of(b->sorted_n[q]) == size && wide_of(b->sorted_n[q]) == wide) ++q;
+    auto tube = [&](const TubeLaunch &l) {
         cudaStream_t st = used < 6 ? b->aux[used] : b->stream;
-        if (used < 6) e = cudaStreamWaitEvent(st, b->fork, 0);
-        if (e == cudaSuccess)
-            e = b->precision == CUMC_FP32 ? launch_tube_fp32(b->d, b->recon, b->riemann, p, q - p, size, wide, st)
-                                          : launch_tube_fp64(b->d, b->recon, b->riemann, p, q - p, size, wide, st);
-        if (e != cudaSuccess && size == 16 && p == big) {
-            cudaGetLastError();  // no room for a 16-CTA cluster: these are the largest, a prefix
-            big = p = q;
-            e = cudaSuccess;
-            continue;
+        cudaError_t r = used < 6 ? cudaStreamWaitEvent(st, b->fork, 0) : cudaSuccess;
+        if (r == cudaSuccess)
+            r = b->precision == CUMC_FP32 ? launch_tube_fp32(b->d, b->recon, b->riemann, l.first, l.count, l.size, l.wide, st)
+                                          : launch_tube_fp64(b->d, b->recon, b->riemann, l.first, l.count, l.size, l.wide, st);
+        if (r != cudaSuccess) {
+            cudaGetLastError();
+            return false;
         }
         b->launches++;
-        if (used < 6 && e == cudaSuccess) {
-            e = cudaEventRecord(b->join[used], st);
-            ++used;
+        if (used < 6) {
+            const cudaError_t w = cudaEventRecord(b->join[used++], st);
+            if (e == cudaSuccess) e = w;
         }
-        p = q;
-    }
-    if (e == cudaSuccess && big > 0) e = run_persistent(b, big);
+        return true;
+    };
+    run_plan(tube_plan(b->sorted_n, b->sm_count), tube, [&](int first, int count) {
+        if (e == cudaSuccess) e = run_persistent(b, first, count);
+        return e == cudaSuccess;
+    });
     for (int i = 0; i < used; ++i) {
         const cudaError_t w = cudaStreamWaitEvent(b->stream, b->join[i], 0);
         if (e == cudaSuccess) e = w;
@@ -307,7 +275,7 @@ int cumc_batch_run(cumc_batch *b, int max_steps, double *t_out, int *steps_out, 
     if (!b) return bfail(b, CUMC_EINVAL, "null batch");
     b->d.max_steps = max_steps > 0 ? max_steps : 0x7fffffff;
     // cumc_batch_set_cluster's shape belongs to the persistent kernel
-    const cudaError_t e = b->coop_min_n < 0 ? run_tubes(b) : run_persistent(b, b->nprob);
+    const cudaError_t e = b->coop_min_n < 0 ? run_tubes(b) : run_persistent(b, 0, b->nprob);
     if (e != cudaSuccess) return bfail(b, CUMC_ECUDA, std::string("batch launch: ") + cudaGetErrorString(e));
     if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(b->stream) != cudaSuccess)
         return bfail(b, CUMC_ECUDA, "batch kernel failed");
