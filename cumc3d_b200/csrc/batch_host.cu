@@ -232,12 +232,13 @@ static cudaError_t run_persistent(cumc_batch *b, int first, int count) {
 // The batch as tube_plan.h lays it out, each class of clusters on a stream of its
 // own, the largest first.
 static cudaError_t run_tubes(cumc_batch *b) {
-    if (!b->fork) {
-        cudaError_t e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
+    if (!b->fork) {  // created last: a run that failed half way is taken up again here
+        cudaError_t e = cudaSuccess;
         for (int i = 0; i < 6 && e == cudaSuccess; ++i) {
-            e = cudaStreamCreateWithFlags(&b->aux[i], cudaStreamNonBlocking);
-            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join[i], cudaEventDisableTiming);
+            if (!b->aux[i]) e = cudaStreamCreateWithFlags(&b->aux[i], cudaStreamNonBlocking);
+            if (e == cudaSuccess && !b->join[i]) e = cudaEventCreateWithFlags(&b->join[i], cudaEventDisableTiming);
         }
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
         if (e != cudaSuccess) return e;
     }
     cudaError_t e = cudaEventRecord(b->fork, b->stream);
