@@ -1787,16 +1787,27 @@ int cumc_create(const cumc_config *cfg, cumc_handle **out) {
         d.QL[i] = a;
         d.QR[i] = b;
     }
-    A(d.EX, N3); A(d.EY, N3); A(d.EZ, N3);
+    // edge EMFs, one block
+    double *edges = nullptr;
+    const size_t edge_stride = ((size_t)N3 + 31) & ~(size_t)31;
+    A(edges, 3 * edge_stride);
+    d.EX = edges;
+    d.EY = edges ? edges + edge_stride : nullptr;
+    d.EZ = edges ? edges + 2 * edge_stride : nullptr;
     // (up to 131072 cells the list's launch costs a stage more than it saves)
     if ((long long)nx * ny * nz > 131072 && cfg->precision == CUMC_FP64 && cfg->riemann == CUMC_RS_HLLD) {
-        // the list of deferred faces: one cell in 4 (34 B a cell, 5% of a
-        // handle), at least 256; the spherical torus fills 0.07 a cell
-        d.fix_cap = (unsigned)(N3 / 4 > 256 ? N3 / 4 : 256);
-        A(d.fix, (size_t)16 * d.fix_cap);
+        // The list of deferred faces lies on the edge EMFs, which are dead from the
+        // update of one stage to k_edge of the next, so it costs no memory: 132 B a
+        // face, one padded cell in 5.5; the spherical torus fills 0.07 a cell.  The
+        // update of the index-0 layers also reads edges outside 0..n, which only
+        // reach face fields that the recovery replaces -- but not on a slab's lower
+        // cut plane, so a slab has a list of its own.
+        double *list = edges;
+        d.fix_cap = (unsigned)(2 * 3 * edge_stride / 33);
+        if (zcut[0]) A(list, 3 * edge_stride);
+        d.fix = list;
+        d.fix_at = list ? (unsigned *)(list + (size_t)16 * d.fix_cap) : nullptr;
         double *q = nullptr;
-        A(q, d.fix_cap / 2 + 2);
-        d.fix_at = (unsigned *)q;
         A(q, 1);
         d.fix_n = (unsigned *)q;
     }
