@@ -1127,6 +1127,104 @@ __global__ void k_dv_check(unsigned long long seed, long long n, unsigned long l
     if (bad) atomicAdd(mismatch, bad);
 }
 
+// The quotients and roots of fast64.cuh against the IEEE operators over the
+// ranges its callers accept.  what: 0 quo, 1 quo with a negative divisor, 2
+// sqrt64, 3 third64; a quarter of the mantissas are powers of two, short, or a
+// few ulps from 1 or 2.  4, 5: quotients built to lie within 4 x 2^-54 ulp of a
+// rounding boundary, the divisors' mantissas up to 1.99, or all; 6: roots built to
+// lie within 2^-34 ulp of one.
+__device__ __forceinline__ double check_mantissa(unsigned long long z, int e, bool divisor) {
+    unsigned long long m = z & 0x000FFFFFFFFFFFFFull;
+    switch ((z >> 52) & 15) {
+        case 0: m = 0; break;
+        case 1: m = m & 0xFF; break;                                // just above a power of two
+        case 2: m = 0x000FFFFFFFFFFFFFull - (m & 0xFF); break;      // just below the next
+        case 3: m = m & 0x000FF00000000000ull; break;               // short
+    }
+    if (divisor && (m & 0xFFFFFFFFull) == 0xFFFFFFFFull) m ^= 1ull;  // the tests exclude such a divisor
+    return __longlong_as_double((long long)(((unsigned long long)(1023 + e) << 52) | m));
+}
+// x, b with x / b = (half an ulp off a representable number) +- k 2^-54 ulp, b odd
+__device__ __forceinline__ bool check_hard_quotient(unsigned long long z, unsigned long long z2, bool all, double &x, double &b) {
+    unsigned long long bi = (z >> 12) | (1ull << 52) | 1ull;
+    if (!all && bi > 0x1FD70A3D70A3D7ull) bi -= 1ull << 51;          // 1.99 x 2^52
+    const int k = 1 + 2 * (int)((z2 >> 1) & 3);
+    unsigned long long t = (z2 & 1) ? (unsigned long long)k : bi - (unsigned long long)k;
+    for (int s = 0; s < 54; ++s) t = (t & 1) ? (t >> 1) + (bi >> 1) + 1 : (t >> 1);  // k 2^-54 mod b
+    if (t == 0) return false;
+    while (t < (1ull << 52)) t <<= 1;
+    b = (double)bi;
+    x = (double)t;
+    return not_ones(b);
+}
+// x with sqrt(x) = M + 1/2 + (c - 1/4) / (2 M + 1) in units of the result's ulp,
+// |c| <= 400000: M from a square root of 1 - 4 c modulo a power of two
+__device__ __forceinline__ bool check_hard_root(long long i, double &x) {
+    const int odd = (int)(i & 1), sel = (int)(i >> 1) & 3;
+    const long long c = 2 * ((i >> 3) % 400001) - 400000;
+    if (c == 0) return false;
+    const int K = odd ? 56 : 55, sh = odd ? 54 : 53;
+    const unsigned long long a = (unsigned long long)(1 - 4 * c);
+    if ((a & 7) != 1) return false;
+    unsigned long long w = 1;
+    for (int bit = 3; bit < K; ++bit)
+        if (((w * w - a) >> bit) & 1) w += 1ull << (bit - 1);
+    const unsigned long long half = 1ull << (K - 1), mask = (1ull << K) - 1;
+    if (sel & 1) w = 0ull - w;
+    if (sel & 2) w += half;
+    w &= mask;
+    const unsigned long long M = ((w - 1) / 2) & ((1ull << 53) - 1);
+    if (M < (1ull << 52)) return false;
+    const unsigned __int128 X = (unsigned __int128)M * (M + 1) + (__int128)c;
+    if ((unsigned long long)X & ((1ull << sh) - 1)) return false;
+    const unsigned __int128 xi = X >> sh;
+    if ((xi >> 53) != 0) return false;
+    x = ldexp((double)(unsigned long long)xi, sh - 104);
+    return true;
+}
+__global__ void k_fast64_check(int what, unsigned long long seed, long long n, unsigned long long *mismatch,
+                               double *example) {
+    long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    unsigned long long bad = 0;
+    for (; i < n; i += stride) {
+        const unsigned long long z1 = mix64(seed + (unsigned long long)i * 0x9E3779B97F4A7C15ull);
+        const unsigned long long z2 = mix64(z1 ^ 0xD1B54A32D192ED03ull);
+        const unsigned long long z3 = mix64(z2 + 0x8CB92BA72F3D8DD7ull);
+        double x = 1.0, b = 1.0, ref, got;
+        if (what <= 1) {
+            const int eb = (int)(z3 % 603) - 133;                   // 2^-133 .. 2^470
+            int ex = eb + (int)((z3 >> 16) % 1161) - 960;           // quotients 2^-960 .. 2^200
+            if (ex < -960) ex = -960;
+            b = check_mantissa(z2, eb, true);
+            x = (z3 >> 48) % 64 == 0 ? 0.0 : check_mantissa(z1, ex, false);
+            if ((z3 >> 60) & 1) x = -x;
+            if (what == 1) b = -b;
+            ref = x / b;
+            got = what == 0 ? quo<true>(x, b, inv64(b)) : quo<false>(x, b, inv64(b));
+        } else if (what == 2 || what == 6) {
+            if (what == 2) x = check_mantissa(z1, (int)(z3 % 1300) - 400, false);
+            else if (!check_hard_root(i, x)) continue;
+            ref = sqrt(x);
+            got = sqrt64(x);
+        } else if (what == 3) {
+            x = check_mantissa(z1, (int)(z3 % 1867) - 967, false);
+            if ((z3 >> 60) & 1) x = -x;
+            ref = x / 3.0;
+            got = third64(x);
+        } else {
+            if (!check_hard_quotient(z1, z2, what == 5, x, b)) continue;
+            ref = x / b;
+            got = quo<true>(x, b, inv64(b));
+        }
+        if (__double_as_longlong(ref) != __double_as_longlong(got)) {
+            if (bad == 0) { example[0] = x; example[1] = b; }
+            ++bad;
+        }
+    }
+    if (bad) atomicAdd(mismatch, bad);
+}
+
 // FP64 pipe probe: independent DFMA chains, 8 per thread, no memory traffic
 __global__ void k_dfma_probe(double *out, int iters) {
     double a[8];
@@ -2948,6 +3046,25 @@ int cumc_check_dv(unsigned long long seed, long long n, unsigned long long *mism
     cudaMemset(m, 0, sizeof(*m));
     cudaMemset(ex, 0, 2 * sizeof(*ex));
     k_dv_check<<<148 * 16, 256>>>(seed, n, m, ex);
+    cudaError_t e = cudaDeviceSynchronize();
+    cudaMemcpy(mismatches, m, sizeof(*m), cudaMemcpyDeviceToHost);
+    cudaMemcpy(example, ex, 2 * sizeof(*ex), cudaMemcpyDeviceToHost);
+    cudaFree(m);
+    cudaFree(ex);
+    return e == cudaSuccess ? CUMC_OK : CUMC_ECUDA;
+}
+
+int cumc_check_fast64(int what, unsigned long long seed, long long n, unsigned long long *mismatches, double *example) {
+    if (what < 0 || what > 6 || !mismatches || !example) return CUMC_EINVAL;
+    unsigned long long *m = nullptr;
+    double *ex = nullptr;
+    if (cudaMalloc(&m, sizeof(*m)) != cudaSuccess || cudaMalloc(&ex, 2 * sizeof(*ex)) != cudaSuccess) {
+        cudaFree(m);
+        return CUMC_ECUDA;
+    }
+    cudaMemset(m, 0, sizeof(*m));
+    cudaMemset(ex, 0, 2 * sizeof(*ex));
+    k_fast64_check<<<148 * 16, 256>>>(what, seed, n, m, ex);
     cudaError_t e = cudaDeviceSynchronize();
     cudaMemcpy(mismatches, m, sizeof(*m), cudaMemcpyDeviceToHost);
     cudaMemcpy(example, ex, 2 * sizeof(*ex), cudaMemcpyDeviceToHost);

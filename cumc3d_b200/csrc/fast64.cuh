@@ -18,11 +18,12 @@
 // one fused multiply-add (Markstein, IBM J. Res. Dev. 34, 1990); square root
 // by one third-order step on x^(-1/2) and the same kind of residual
 // correction.  The seed is good to 2^-19.9, so y is within 0.51 ulp of 1/b.
-// Measured against x / y and sqrt(x): no difference in 2^32 random pairs.  On
+// Measured against x / y and sqrt(x) (cumc_check_fast64): no difference in 2^30
+// generated pairs or arguments of the ranges used here.  On
 // pairs built so that the quotient lies within 2^-52 ulp of a rounding
 // boundary (7 of 2^28) the quotient can fall on the other side when the
-// divisor's mantissa is above 1.99; the chance for an arbitrary pair is below
-// 2^-70.  Power-of-two numerators over an all-ones divisor, the one case that
+// divisor's mantissa is above 1.99 (none below); the chance for an arbitrary pair
+// is below 2^-70.  Power-of-two numerators over an all-ones divisor, the one case that
 // occurs in practice (1 / 0.999...), are excluded by the tests.
 #pragma once
 #include "mhd_device.cuh"

@@ -22,6 +22,7 @@ EXPORTS = [
     "cumc_initial_update", "cumc_finddt", "cumc_rk3_step", "cumc_evolve", "cumc_max_divb",
     "cumc_sync", "cumc_launch_count", "cumc_stream", "cumc_profile_step", "cumc_fp64_peak", "cumc_autotune",
     "cumc_set_tuning", "cumc_set_concurrent_sweeps", "cumc_fallback_count", "cumc_check_div3", "cumc_check_dv",
+    "cumc_check_fast64",
     "cumc_batch_create", "cumc_batch_destroy", "cumc_batch_set_state", "cumc_batch_get_state",
     "cumc_batch_run", "cumc_batch_sync", "cumc_batch_stream", "cumc_batch_launch_count", "cumc_batch_last_error",
     "cumc_batch_set_cluster",
@@ -79,6 +80,7 @@ def load_library(path=None):
     L.cumc_set_concurrent_sweeps.argtypes = [C.c_void_p, C.c_int]
     L.cumc_fallback_count.argtypes = [C.c_void_p, C.c_int, C.POINTER(C.c_ulonglong)]
     L.cumc_check_div3.argtypes = [C.c_ulonglong, C.c_longlong, C.POINTER(C.c_ulonglong), C.POINTER(C.c_double)]
+    L.cumc_check_fast64.argtypes = [C.c_int, C.c_ulonglong, C.c_longlong, C.POINTER(C.c_ulonglong), C.POINTER(C.c_double)]
     L.cumc_check_dv.argtypes = [C.c_ulonglong, C.c_longlong, C.POINTER(C.c_ulonglong), C.POINTER(C.c_double)]
     L.cumc_last_error.argtypes = [C.c_void_p]
     L.cumc_last_error.restype = C.c_char_p
@@ -868,4 +870,15 @@ def check_dv(seed, n):
     rc = load_library().cumc_check_dv(seed, n, C.byref(m), ex)
     if rc != 0:
         raise CumcError(rc, "dv check failed to run")
+    return m.value, (ex[0], ex[1])
+
+
+def check_fast64(what, seed, n):
+    """(mismatches, (x, y) of one differing pair) of the branch-free quotients
+    and roots (what: the kinds of cumc_check_fast64) against the IEEE ones."""
+    m = C.c_ulonglong()
+    ex = (C.c_double * 2)()
+    rc = load_library().cumc_check_fast64(what, seed, n, C.byref(m), ex)
+    if rc != 0:
+        raise CumcError(rc, "fast64 check failed to run")
     return m.value, (ex[0], ex[1])

@@ -241,6 +241,16 @@ int cumc_check_div3(unsigned long long seed, long long n, unsigned long long *mi
  * example[0..1] = one differing pair. */
 int cumc_check_dv(unsigned long long seed, long long n, unsigned long long *mismatches, double *example);
 
+/* Numerics self-check (no counterpart in the reference): the branch-free
+ * quotients and roots of the FP64 WENO-Z, HLLD, update and recovery against
+ * x / y, sqrt(x) and x / 3 on n generated operands of the ranges they are used
+ * for.  what: 0 quotients, 1 the same with negative divisors, 2 square roots, 3
+ * thirds, 4 quotients built to lie within 2^-52 ulp of a rounding boundary with
+ * divisors whose mantissa is at most 1.99, 5 the same with any divisor (a few
+ * in 2^28 of these round the other way), 6 square roots built to lie close to
+ * one.  *mismatches counts differing bit patterns, example[0..1] = one pair. */
+int cumc_check_fast64(int what, unsigned long long seed, long long n, unsigned long long *mismatches, double *example);
+
 /* Measured FP64 fused-multiply-add throughput of the current device in
  * TFLOP/s (the denominator of the FP64-pipe roofline). */
 int cumc_fp64_peak(double *tflops);
