@@ -2318,6 +2318,17 @@ int cumc_set_tuning(cumc_handle *h, const int *choice) {
     return CUMC_OK;
 }
 
+int cumc_deferred_faces(cumc_handle *h, unsigned *most, unsigned *capacity) {
+    if (!h || !most || !capacity) return fail(h, CUMC_EINVAL, "null argument");
+    *most = 0;
+    *capacity = h->d.fix_n ? h->d.fix_cap : 0;
+    if (!h->d.fix_n) return CUMC_OK;
+    CK(cudaMemcpyAsync(most, h->d.fix_n + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaMemsetAsync(h->d.fix_n + 1, 0, sizeof(unsigned), h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    return CUMC_OK;
+}
+
 int cumc_fallback_count(cumc_handle *h, int enable, unsigned long long *count_out) {
     if (!h) return fail(h, CUMC_EINVAL, "null handle");
     if (enable < -1 || enable > 1) return fail(h, CUMC_EINVAL, "enable must be -1, 0 or 1");

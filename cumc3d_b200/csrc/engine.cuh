@@ -73,7 +73,8 @@ struct Dev {
     void *QL[7], *QR[7];   // face states of the split flux path (double or float)
 
     // faces of the FP64 HLLD form left to k_faces_deferred: their two states
-    // (16 arrays of fix_cap), 3 * cell + direction, and how many
+    // (16 arrays of fix_cap), 3 * cell + direction, and how many (fix_n[0]; [1]:
+    // the most of any stage, those beyond fix_cap included)
     double *fix;
     unsigned *fix_at, *fix_n;
     unsigned fix_cap;

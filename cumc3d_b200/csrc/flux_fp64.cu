@@ -13,7 +13,8 @@ void launch_flux_fp64(const Dev &d, int dir, int rec, int rs, dim3 grid, dim3 bl
 __global__ void __launch_bounds__(128) k_faces_deferred(const Dev d) {
     pdl_wait();
     if (d.S->done) return;
-    const unsigned n = *d.fix_n < d.fix_cap ? *d.fix_n : d.fix_cap;
+    const unsigned all = *d.fix_n, n = all < d.fix_cap ? all : d.fix_cap;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && all > d.fix_n[1]) d.fix_n[1] = all;  // cumc_deferred_faces
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double q[17], f[9];
 #pragma unroll

@@ -22,7 +22,7 @@ EXPORTS = [
     "cumc_initial_update", "cumc_finddt", "cumc_rk3_step", "cumc_evolve", "cumc_max_divb",
     "cumc_sync", "cumc_launch_count", "cumc_stream", "cumc_profile_step", "cumc_fp64_peak", "cumc_autotune",
     "cumc_set_tuning", "cumc_set_concurrent_sweeps", "cumc_fallback_count", "cumc_check_div3", "cumc_check_dv",
-    "cumc_check_fast64",
+    "cumc_check_fast64", "cumc_deferred_faces",
     "cumc_batch_create", "cumc_batch_destroy", "cumc_batch_set_state", "cumc_batch_get_state",
     "cumc_batch_run", "cumc_batch_sync", "cumc_batch_stream", "cumc_batch_launch_count", "cumc_batch_last_error",
     "cumc_batch_set_cluster",
@@ -79,6 +79,7 @@ def load_library(path=None):
     L.cumc_set_tuning.argtypes = [C.c_void_p, C.POINTER(C.c_int)]
     L.cumc_set_concurrent_sweeps.argtypes = [C.c_void_p, C.c_int]
     L.cumc_fallback_count.argtypes = [C.c_void_p, C.c_int, C.POINTER(C.c_ulonglong)]
+    L.cumc_deferred_faces.argtypes = [C.c_void_p, C.POINTER(C.c_uint), C.POINTER(C.c_uint)]
     L.cumc_check_div3.argtypes = [C.c_ulonglong, C.c_longlong, C.POINTER(C.c_ulonglong), C.POINTER(C.c_double)]
     L.cumc_check_fast64.argtypes = [C.c_int, C.c_ulonglong, C.c_longlong, C.POINTER(C.c_ulonglong), C.POINTER(C.c_double)]
     L.cumc_check_dv.argtypes = [C.c_ulonglong, C.c_longlong, C.POINTER(C.c_ulonglong), C.POINTER(C.c_double)]
@@ -248,6 +249,14 @@ class Solver:
         n = C.c_ulonglong()
         self._check(self.L.cumc_fallback_count(self.h, int(enable), C.byref(n)))
         return int(n.value)
+
+    def deferred_faces(self):
+        """(most, capacity): the most faces of the FP64 HLLD form that one stage
+        has left to the plain solver since the last call, and how many the
+        handle's list holds (0: no list, none counted)."""
+        most, cap = C.c_uint(), C.c_uint()
+        self._check(self.L.cumc_deferred_faces(self.h, C.byref(most), C.byref(cap)))
+        return int(most.value), int(cap.value)
 
     # ---- learned smooth-face flag (FP32 WENO form, handle created with learned=1) ----
     def learn_set(self, params, threshold=0.0, audit_interval=10, audit_tol=1e-6, flag_interval=1):

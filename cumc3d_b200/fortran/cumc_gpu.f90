@@ -314,6 +314,11 @@ INTERFACE
     INTEGER(C_INT), VALUE :: enable
     INTEGER(C_LONG_LONG), INTENT(OUT) :: count_out
   END FUNCTION
+  INTEGER(C_INT) FUNCTION cumc_deferred_faces(h, most, capacity) BIND(C, NAME='cumc_deferred_faces')
+    IMPORT :: C_INT, C_PTR
+    TYPE(C_PTR), VALUE :: h
+    INTEGER(C_INT), INTENT(OUT) :: most, capacity
+  END FUNCTION
   INTEGER(C_INT) FUNCTION cumc_check_dv(seed, n, mismatches, example) BIND(C, NAME='cumc_check_dv')
     IMPORT :: C_INT, C_LONG_LONG, C_DOUBLE
     INTEGER(C_LONG_LONG), VALUE :: seed, n

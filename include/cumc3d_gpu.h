@@ -229,6 +229,13 @@ int cumc_set_concurrent_sweeps(cumc_handle *h, int on);
  * fallback cell and nothing otherwise. */
 int cumc_fallback_count(cumc_handle *h, int enable, unsigned long long *count_out);
 
+/* Faces of the FP64 HLLD form that the fast solver did not vouch for (no
+ * counterpart in the reference): *most = the most that any one stage has left
+ * to the plain solver since the last call, *capacity = how many of them the
+ * handle's list holds (the rest are solved in place; 0: no list, all in place
+ * and none counted).  Synchronises the handle's stream. */
+int cumc_deferred_faces(cumc_handle *h, unsigned *most, unsigned *capacity);
+
 /* Numerics self-check (no counterpart in the reference): compares the FP64
  * engine's FMA-corrected division by 3 with the IEEE quotient on n generated
  * normal inputs; *mismatches counts differing bit patterns. */
