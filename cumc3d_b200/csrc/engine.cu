@@ -1885,24 +1885,30 @@ int cumc_create(const cumc_config *cfg, cumc_handle **out) {
         d.QL[i] = a;
         d.QR[i] = b;
     }
+    // (up to 131072 cells the list's launch costs a stage more than it saves)
+    const bool deferred =
+        (long long)nx * ny * nz > 131072 && cfg->precision == CUMC_FP64 && cfg->riemann == CUMC_RS_HLLD;
     // edge EMFs, one block
     double *edges = nullptr;
     const size_t edge_stride = ((size_t)N3 + 31) & ~(size_t)31;
-    A(edges, 3 * edge_stride);
+    const size_t edge_room = deferred && d.coord == 2 ? 33 * (edge_stride / 8) : 3 * edge_stride;
+    A(edges, edge_room);
     d.EX = edges;
     d.EY = edges ? edges + edge_stride : nullptr;
     d.EZ = edges ? edges + 2 * edge_stride : nullptr;
-    // (up to 131072 cells the list's launch costs a stage more than it saves)
-    if ((long long)nx * ny * nz > 131072 && cfg->precision == CUMC_FP64 && cfg->riemann == CUMC_RS_HLLD) {
+    if (deferred) {
         // The list of deferred faces lies on the edge EMFs, which are dead from the
-        // update of one stage to k_edge of the next, so it costs no memory: 132 B a
-        // face, one padded cell in 5.5; the spherical torus fills 0.07 a cell.  The
-        // update of the index-0 layers also reads edges outside 0..n, which only
-        // reach face fields that the recovery replaces -- but not on a slab's lower
-        // cut plane, so a slab has a list of its own.
+        // update of one stage to k_edge of the next: 132 B a face, room for 0.18 of
+        // them a padded cell.  The most any stage left there, faces per cell:
+        // 0.055 on the cylindrical torus, 0.018 on the blast, 0.31 (PPM) and 0.35
+        // (WENO-Z) on the spherical torus, whose block holds 0.25 a padded cell
+        // (1.5% of a handle; with 0.18 the first 24 steps at 62 x 50 x 64 took 590
+        // us against 573).  The update of the index-0 layers also reads edges
+        // outside 0..n, which only reach face fields that the recovery replaces --
+        // but not on a slab's lower cut plane, so a slab has a list of its own.
         double *list = edges;
-        d.fix_cap = (unsigned)(2 * 3 * edge_stride / 33);
-        if (zcut[0]) A(list, 3 * edge_stride);
+        d.fix_cap = (unsigned)(2 * edge_room / 33);
+        if (zcut[0]) A(list, edge_room);
         d.fix = list;
         d.fix_at = list ? (unsigned *)(list + (size_t)16 * d.fix_cap) : nullptr;
         double *q = nullptr;
