@@ -1885,9 +1885,16 @@ int cumc_create(const cumc_config *cfg, cumc_handle **out) {
         d.QL[i] = a;
         d.QR[i] = b;
     }
-    // (up to 131072 cells the list's launch costs a stage more than it saves)
+    // Which handles have a list of deferred faces.  Its launch costs 3 to 10 us a
+    // step (blast WENO-Z 40^3 216 -> 224, 50^3 385 -> 388, cylindrical torus 48 x 32 x 64
+    // PPM 249 -> 259, 60 x 50 x 60 WENO-Z 484 -> 487); what it saves grows with the faces deferred:
+    // spherical torus PPM, without and with: 48 x 24 x 40 206 / 209, 56 x 28 x 40 323 / 301
+    // (276 / 278 after 1500 steps), 62 x 32 x 40 387 / 335 (348 / 318), 62 x 44 x 64 649 / 563.
+    // There the limited reconstructions keep leaving 0.2 faces a cell, WENO-Z 0.02
+    // (62 x 32 x 40 315 / 322); elsewhere fewer.
+    const long long list_from = d.coord == 2 && cfg->recon != CUMC_RECON_WENO ? 70000 : 131072;
     const bool deferred =
-        (long long)nx * ny * nz > 131072 && cfg->precision == CUMC_FP64 && cfg->riemann == CUMC_RS_HLLD;
+        (long long)nx * ny * nz > list_from && cfg->precision == CUMC_FP64 && cfg->riemann == CUMC_RS_HLLD;
     // edge EMFs, one block
     double *edges = nullptr;
     const size_t edge_stride = ((size_t)N3 + 31) & ~(size_t)31;

@@ -98,7 +98,7 @@ __device__ __forceinline__ void store_face(const Dev &d, int ci, const T *fo) {
 
 // Solve the face at ci and store it.  A face that hlld64 does not vouch for
 // goes on the stage's list, which k_faces_deferred works off after the sweeps:
-// about one face in a hundred where fields decay towards zero (products
+// one face in ten to one in a hundred where fields decay towards zero (products
 // between 1e-323 and 1e-271), but spread so that the plain form inside this
 // kernel ran in most warps (spherical torus 124 x 44 x 128, the three sweeps
 // of a step: 1.42 ms that way, 0.86 with the list).  Without a list

@@ -89,3 +89,23 @@ def test_no_list_on_a_small_grid():
     s = Solver(spec)
     assert s.deferred_faces() == (0, 0)
     s.close()
+
+
+@pytest.mark.parametrize("recon", ["ppm", "tvdmm"])
+def test_spherical_torus_below_the_general_size(oracle_mod, recon):
+    """84,320 cells, whose limited reconstruction leaves many faces for good."""
+    from cumc3d_b200.engine import Solver
+    spec, prim, eps = models.torus_sph(nr=62, ntheta=34, nphi=40, recon=recon)
+    spec["fix_periodic_normal_faces"] = 1
+    spec["positivity_fallback"] = 1
+    s, o = Solver(spec), oracle_mod.Oracle(spec)
+    for q in (s, o):
+        q.set_state(prim, eps)
+        q.initial_update()
+    assert s.evolve(1e30, 20) == o.evolve(1e30, 20)
+    most, capacity = s.deferred_faces()
+    assert 0.1 * 84320 < most <= capacity
+    (p, e), (po, eo) = s.get_state(), o.get_state()
+    assert_bitwise(dict(prim=p, eps=e), dict(prim=po, eps=eo), spec, what=("prim", "eps"))
+    s.close()
+    o.close()
