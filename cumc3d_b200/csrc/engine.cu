@@ -1717,14 +1717,18 @@ static int check_scalars(cumc_handle *h) {
     return CUMC_OK;
 }
 
-// Whether a handle's stage kernels are launched programmatically dependent.
-// 64^3 PPM 486 -> 467 us a step, 101 x 96 x 90 1379 -> 1354; below they cost
-// (24^3 128 -> 161, 64^2 104 -> 124).  Only where the launch before on the same
-// stream is the kernel a stage kernel depends on: not with concurrent sweeps,
+// Whether a handle's stage kernels are launched programmatically dependent: from
+// 100,000 cells up (padded cells would count a plane sevenfold).  Us a step, off
+// and on: blast WENO-Z 36^3 201 / 207, 42^3 260 / 258, 46^3 289 / 280, 50^3 385 / 379,
+// 64^3 587 / 572; waves PPM 42^3 229 / 225, 50^3 288 / 281; cylindrical torus
+// 48 x 32 x 32 228 / 241, 64 x 40 x 50 359 / 353; spherical 62 x 36 x 44 423 / 432,
+// 62 x 40 x 48 500 / 490; vortex 256^2 233 / 247, 300^2 286 / 288, 350^2 351 / 342, 600^2
+// 837 / 825; tube 5000 105 / 109, 120000 1065 / 1056.  Only where the launch before on the
+// same stream is the kernel a stage kernel depends on: not with concurrent sweeps,
 // whose join has several predecessors, and not for a slab, whose exchange puts
 // copies and waits on its neighbours' streams between two kernels twice a stage.
 static int programmatic(const Dev &d, bool concurrent) {
-    return d.N3 >= 200000 && !concurrent && !d.zcut[0] && !d.zcut[1] ? 1 : 0;
+    return (long long)d.nx * d.ny * d.nz >= 100000 && !concurrent && !d.zcut[0] && !d.zcut[1] ? 1 : 0;
 }
 
 extern "C" {
