@@ -95,6 +95,7 @@ constexpr int GHOST_BZ = 10;     // P 7, the z face field
 // an array a fill leaves out (the normal face field) keeps its index there.
 // No source is itself written: on every axis that moves it is an interior index.
 // Three dependent passes and the clamps took four launches a stage.
+template <int SLAB>
 __global__ void __launch_bounds__(256) k_ghosts(const Dev d, const GhostList gl) {
     pdl_wait();
     if (d.S->done) return;
@@ -127,8 +128,8 @@ __global__ void __launch_bounds__(256) k_ghosts(const Dev d, const GhostList gl)
     // a z side shared with a neighbouring slab is filled by the exchange; at the
     // seam of a ring that leaves out the normal field where the z fill does
     // (halo_arrays), and its x and y ghosts are filled here as on any plane
-    const int cut = l < 1 ? d.zcut[0] : l > d.nz ? d.zcut[1] : 0;
-    if (cut && (cut == 1 || d.fixn)) return;
+    const int cut = !SLAB ? 0 : l < 1 ? d.zcut[0] : l > d.nz ? d.zcut[1] : 0;
+    if (cut && (cut == 1 || d.fixn || blockIdx.y != 2)) return;
     const int c = cidx(d, j, k, l);
     int side[3], off[3];
     {
@@ -143,7 +144,7 @@ __global__ void __launch_bounds__(256) k_ghosts(const Dev d, const GhostList gl)
             off[x] = (ghost_src(d.bf[side[x]], s == 0, s == 0 ? 1 - i3[x] : i3[x] - n3[x], n3[x]) - i3[x]) * st[x];
         }
     }
-    const int first = blockIdx.y < 2 ? 4 * blockIdx.y : blockIdx.y == 2 ? 8 : 11;
+    const int first = cut ? GHOST_BZ : blockIdx.y < 2 ? 4 * blockIdx.y : blockIdx.y == 2 ? 8 : 11;
     const int last = blockIdx.y < 2 ? first + 4 : blockIdx.y == 2 ? 11 : 13;
     double v[4];
     bool moved[4];
@@ -152,7 +153,7 @@ __global__ void __launch_bounds__(256) k_ghosts(const Dev d, const GhostList gl)
         const int m = first + q;
         v[q] = 0.0;
         moved[q] = false;
-        if (m >= last || (cut && m != GHOST_BZ)) continue;
+        if (m >= last) continue;
         int o = 0;
 #pragma unroll
         for (int x = 0; x < 3; ++x)
@@ -1549,7 +1550,9 @@ static void launch_ghosts(cumc_handle *h) {
     add(d.CS, 1, 7);  // FINDPRESSURE output, even (recomputed identically by the reference)
     add(d.EPS, 1, 7);
     const long long cells = 6LL * d.NY * d.NZ + 6LL * d.nx * d.NZ + 6LL * d.nx * d.ny;
-    launch(k_ghosts, dim3((unsigned)((cells + 255) / 256), GHOST_GROUPS), 256, 0, h->stream, d.pdl, d, g);
+    const dim3 grid((unsigned)((cells + 255) / 256), GHOST_GROUPS);
+    if (d.zcut[0] || d.zcut[1]) launch(k_ghosts<1>, grid, 256, 0, h->stream, d.pdl, d, g);
+    else launch(k_ghosts<0>, grid, 256, 0, h->stream, d.pdl, d, g);
     h->launches++;
 }
 
