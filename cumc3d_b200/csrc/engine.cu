@@ -1721,17 +1721,20 @@ static int check_scalars(cumc_handle *h) {
 }
 
 // Whether a handle's stage kernels are launched programmatically dependent: from
-// 100,000 cells up (padded cells would count a plane sevenfold).  Us a step, off
-// and on: blast WENO-Z 36^3 201 / 207, 42^3 260 / 258, 46^3 289 / 280, 50^3 385 / 379,
-// 64^3 587 / 572; waves PPM 42^3 229 / 225, 50^3 288 / 281; cylindrical torus
-// 48 x 32 x 32 228 / 241, 64 x 40 x 50 359 / 353; spherical 62 x 36 x 44 423 / 432,
-// 62 x 40 x 48 500 / 490; vortex 256^2 233 / 247, 300^2 286 / 288, 350^2 351 / 342, 600^2
-// 837 / 825; tube 5000 105 / 109, 120000 1065 / 1056.  Only where the launch before on the
-// same stream is the kernel a stage kernel depends on: not with concurrent sweeps,
-// whose join has several predecessors, and not for a slab, whose exchange puts
-// copies and waits on its neighbours' streams between two kernels twice a stage.
-static int programmatic(const Dev &d, bool concurrent) {
-    return (long long)d.nx * d.ny * d.nz >= 100000 && !concurrent && !d.zcut[0] && !d.zcut[1] ? 1 : 0;
+// 80,000 cells up in 1D and 2D, 100,000 in 3D, 131072 in FP32, whose shorter
+// kernels end sooner than the next launch arrives.  (Padded cells would
+// count a plane sevenfold.)  What it changes, us a step off -> on: 2D PPM 220^2
+// +2.8 to +4.3%, 256^2 +0.7 to +1.6%, 300^2 -2.0%, 400^2 -3.0%; 2D FP32 256^2 +3.7%, 300^2
+// 0, 350^2 -3.5%; tube 30000 +0.9%, 60000 -0.9%; 3D FP64 36^3 +3%, 46^3 -3%, 64^3 -2.6%,
+// cylindrical torus 48 x 32 x 32 +5.7%, 64 x 40 x 50 -1.7%, spherical 62 x 36 x 44 +2.1%,
+// 62 x 40 x 48 -2.0%; 3D FP32 48^3 +2.3%, 50^3 +0.4%, 52^3 -2.0%, 56^3 -4.5%.  Only where
+// the launch before on the same stream is the kernel a stage kernel depends on:
+// not with concurrent sweeps, whose join has several predecessors, and not for a
+// slab, whose exchange puts copies and waits on its neighbours' streams between
+// two kernels twice a stage.
+static int programmatic(const Dev &d, bool fp32, bool concurrent) {
+    const long long from = d.n_dim < 3 ? 80000 : fp32 ? 131072 : 100000;
+    return (long long)d.nx * d.ny * d.nz >= from && !concurrent && !d.zcut[0] && !d.zcut[1] ? 1 : 0;
 }
 
 extern "C" {
@@ -1790,7 +1793,7 @@ int cumc_create(const cumc_config *cfg, cumc_handle **out) {
     d.tpb_recon = 256;
     d.tpb_riemann = 128;
     d.riemann_minb = 4;
-    d.pdl = programmatic(d, false);
+    d.pdl = programmatic(d, cfg->precision == CUMC_FP32, false);
     d.gamma = cfg->model.gamma; d.cfl = cfg->cfl;
     d.floor_kind = cfg->model.floor_kind; d.source_kind = cfg->model.source_kind; d.bc_kind = cfg->model.bc_kind;
     d.rho_floor = cfg->model.rho_floor; d.eps_floor = cfg->model.eps_floor; d.p_floor = cfg->model.p_floor;
@@ -2390,7 +2393,7 @@ int cumc_set_concurrent_sweeps(cumc_handle *h, int on) {
         for (int i = 0; i < 3; ++i) CK(cudaEventCreateWithFlags(&h->fev[i], cudaEventDisableTiming));
     }
     h->sweeps_concurrent = on != 0;
-    h->d.pdl = programmatic(h->d, on != 0);
+    h->d.pdl = programmatic(h->d, h->cfg.precision == CUMC_FP32, on != 0);
     // a captured step graph holds the old launch order
     drop_graphs(h);
     return CUMC_OK;
