@@ -2,10 +2,15 @@
 
     python -m cumc3d_b200.build
 
-Three translation units:
-  engine.cu     stage kernels, ghost fills, time loop, C-ABI   (--fmad=false)
-  flux_fp64.cu  fused face-flux kernel, plain FP64 form          (--fmad=false)
-  flux_fp32.cu  fused face-flux kernel, FP32 form                (FMA, fast div/sqrt)
+Nine translation units:
+  engine.cu      stage kernels, ghost fills, time loop, C-ABI    (--fmad=false)
+  flux_fp64.cu   face-flux kernels, plain FP64 form              (--fmad=false)
+  flux_fp32.cu   face-flux kernels, FP32 form                    (FMA, fast div/sqrt)
+  batch_host.cu  the batched 1D engine's C-ABI                   (--fmad=false)
+  batch_fp64.cu, batch_fp32.cu  its kernels in both forms        (as the flux units)
+  noalloc.cu     one 1D problem without device allocations       (--fmad=false)
+  learned.cu     the smooth-face flag's network                  (--fmad=false)
+  poisson.cu     self-gravity of the collapsar model             (--fmad=false)
 --fmad=false keeps every FP64 expression in the reference's rounding order
 (no contraction into fused multiply-adds), which is what makes the plain form
 reproduce the Fortran semantics bit for bit.

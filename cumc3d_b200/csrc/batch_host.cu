@@ -1,6 +1,7 @@
 // batch_host.cu -- C-ABI of the batched 1D engine (cumc_batch_* in
 // include/cumc3d_gpu.h).  Packs many 1D problems of uneven size into one set
-// of device arrays and runs them in one persistent launch (batch_kernel.cuh).
+// of device arrays and runs each on a cluster of its own (tube_kernel.cuh), what
+// does not fit one in a persistent launch (batch_kernel.cuh); tube_plan.h decides.
 #include <algorithm>
 #include <cstring>
 #include <numeric>

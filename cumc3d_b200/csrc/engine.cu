@@ -4,7 +4,10 @@
 // One RK stage of the reference (solver/mhd/rungekutta.f90:61-100) is issued
 // as the kernel sequence
 //
-//   k_flux x/y/z        recon + EOS + BUILDSTATES + Riemann + MHD_FLUX      (flux_kernel.cuh)
+//   k_recon, k_riemann  recon + EOS + BUILDSTATES + Riemann + MHD_FLUX of
+//     or k_flux x/y/z   each sweep, in two kernels or one                   (flux_kernel.cuh, recon_tile.cuh)
+//   k_faces_deferred    the faces hlld64 does not vouch for, on handles with
+//                       a list of them                                      (flux_fp64.cu)
 //   k_edge              the 1D/2D face-EMF fill, BOUNDARY_EFIELD and the
 //                       edge EMFs (GS05 arithmetic average)                 (mhd_module.f90:314-432,
 //                                                                            478-840)
@@ -19,10 +22,12 @@
 //                                                                            mhd_module.f90:310-312)
 //   k_ghosts            BOUNDARY (prim, bcell, epsilon, p, c_s) and the
 //                       torus models' CUSTOM_BOUNDARY_X/Z                    (boundary.f90:5-770)
+//   k_bh_update         the black hole's growth (collapsar only)             (custom.f90:450-485)
 //
 // FINDDT is a deterministic min-reduction (exact, order independent; inside
-// cumc_evolve by the last stage's k_recover) whose result stays on the device; a whole step is captured once as a CUDA graph
-// and replayed by cumc_evolve.
+// cumc_evolve by the last stage's k_recover) whose result stays on the device.
+// cumc_evolve replays a step captured once as a CUDA graph, cumc_rk3_step its
+// three stages from the third call on.
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -377,7 +382,7 @@ __global__ void k_snapshot_pack(const Dev d, double *__restrict__ out) {
 // quotients (on Cartesian axes the same three serve all).  With a division
 // apiece the arithmetic of this memory-bound kernel took longer than its loads
 // (256^3, FP64: 4.08 ms a step; 3.05 with shared reciprocals and 3 blocks per
-// SM: 168 registers, no spills -- 4, 5 and 6 blocks took 3.81, 4.07, 4.52).
+// SM: 156 registers, no spills -- 4, 5 and 6 blocks took 3.81, 4.07, 4.52).
 struct CellDens {
     Den64 h[3], fa[3], fb[3];
 };
@@ -2148,7 +2153,7 @@ int cumc_rk3_step(cumc_handle *h, double dt) {
         return fail(h, CUMC_ENOTREADY, "the collapsar source needs cumc_poisson_setup first");
     CK(cudaMemcpyAsync(&h->d.S->dt, &dt, sizeof(double), cudaMemcpyHostToDevice, h->stream));
     // a program that steps by itself pays for a captured step once it has taken
-    // two: 24 to 33 launches from the host cost more than such a step runs on a
+    // two: 15 to 33 launches from the host cost more than such a step runs on a
     // small grid
     if (h->eager_steps < 2) {
         ++h->eager_steps;

@@ -499,8 +499,9 @@ static void launch_recon_tile_c(const Dev &d, int rec, cudaStream_t s) {
         const XTail t = x_tail(d, CPT);
         g = dim3(t.tiles + t.tails, 1, d.nz);
     }
-    // blocks per SM: FP64 WENO-Z unrolls to 250 registers where nothing bounds
-    // it; 2 blocks (126 registers) and, as kind 4, 3 blocks (80, 152 B spilled)
+    // Blocks per SM: kind 4 asks for 4 (64 registers for FP64 PPM, 48 in FP32), the
+    // others take the compiler's choice.  FP64 WENO-Z unrolls to 250 registers
+    // where nothing bounds it: 2 blocks (126) and, as kind 4, 3 (80, 152 B spilled)
     constexpr bool W = sizeof(T) == sizeof(double);
     constexpr int M = KIND == 4 ? 4 : 1, MW = !W ? M : KIND == 4 ? 3 : 2;
     switch (rec) {
@@ -512,8 +513,8 @@ static void launch_recon_tile_c(const Dev &d, int rec, cudaStream_t s) {
     }
 }
 // recon_tile: 1, 2 staged tiles with 1 or 2 cells per thread; 4 one cell per
-// thread at 64 registers (4 blocks per SM); 3 (TMA-staged) falls back to 1
-// where no tensor maps are given
+// thread with more blocks per SM; 3 (TMA-staged) falls back to 1 where no tensor
+// maps are given
 template <class T, int DIR, int UNI>
 static void launch_recon_tile(const Dev &d, int rec, cudaStream_t s) {
     if (d.recon_tile == 2) launch_recon_tile_c<T, DIR, UNI, 2, 2>(d, rec, s);

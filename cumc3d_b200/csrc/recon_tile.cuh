@@ -39,8 +39,8 @@ __host__ __device__ inline dim3 recon_tile_grid(const Dev &d, int dir, int cpt) 
 // columns beyond the last whole tile, `rest` wide, go `rows` rows to a block, as
 // many as its threads and its shared memory hold, instead of 8 (x cpt) rows to a
 // block whose other lanes idle.  FP64 WENO-Z, ms a step before and now: 96 x 64 x 96
-// 1.199 and 1.163, 101 x 96 x 90 1.828 and 1.787, 160^3 7.68 and 7.54, 62 x 64 x 64,
-// whose rows are whole tiles, 0.568 and 0.567.
+// 1.207 and 1.171, 101 x 96 x 90 1.838 and 1.787, 160^3 7.49 and 7.36, 256^3 28.15 and
+// 28.09, 62 x 64 x 64, whose rows are whole tiles, 0.571 and 0.571.
 struct XTail {
     int full, rest, rows, tiles, tails;  // whole tiles a row, as above, blocks a plane of either kind
 };
@@ -60,7 +60,7 @@ __host__ __device__ inline XTail x_tail(const Dev &d, int cpt) {
 }
 // Only FP64 WENO-Z, which is bound by the FP64 pipe the idle lanes keep busy: the
 // width known at run time cost FP32 more than that gave (192^3 7.69 -> 7.72), and
-// PPM won 0.6% (128^3) or lost as much (62 x 64 x 64).  Not with the learned flag,
+// PPM gained 0.5% at 101 x 96 x 90 and lost 0.4% at 70 x 61 x 66.  Not with the learned flag,
 // whose warps are indexed by recon_tile_grid.
 template <class T>
 constexpr bool pack_x(int dir, int rec) { return dir == 0 && rec == REC_WENO && sizeof(T) == sizeof(double); }
@@ -194,9 +194,7 @@ __device__ __forceinline__ void recon_tile_cells(const Dev &d, const T *__restri
     }
 }
 
-// MINB: blocks per SM the register budget is sized for (1: the compiler's
-// choice, about 76 registers for FP64 WENO-Z; 4: 64 registers, a third more
-// resident warps)
+// MINB: blocks per SM the register budget is sized for (launch_recon_tile_c)
 template <class T, int DIR, int REC, int UNI, int CPT, int LRN = 0, int MINB = 1>
 __global__ void __launch_bounds__(256, MINB) k_recon_tile(const Dev d, int stage = 0) {
     pdl_wait();
