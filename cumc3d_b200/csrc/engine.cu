@@ -2563,9 +2563,9 @@ int cumc_poisson_solve(cumc_handle *h, int max_iter, double tol, int *iters_out,
     // 1056, 400 the same).  Up to 8 that remain are launched as they are: the rest of
     // a graph would idle longer (5 iterations at 24 x 16 x 16 150 us, 161).
     int st[3] = {1, 0, 0};
-    for (int round = 0; st[1] == 0 && st[0] < max_iter; ++round) {
+    for (int looks = 0; st[1] == 0 && st[0] < max_iter; ++looks) {
         const int left = max_iter - st[0];
-        int graphs = round == 0 ? 1 : round == 1 ? 3 : 4;
+        int graphs = looks == 0 ? 1 : looks == 1 ? 3 : 4;
         if (left <= 8) {
             for (int i = 0; i < left; ++i) launch_sor_iteration(s, st[0] + 1 + i, h->stream);
             h->launches += 2LL * left;
